@@ -1,13 +1,12 @@
 // Tensor-core (tcgen05) forms of the near field, the ACA queries and the stand-alone evaluation.
 //
 // All three kernels are persistent (one CTA per SM, up to ~227 KB shared
-// memory, 512 TMEM columns) and drive the tile engine of tc_mlp.cuh with a
-// stream of 128-evaluation tiles; the epilogue threads compute the features of
-// the next tile before the engine retires the current one:
-//   k_near_tc : close pairs (I, J) fetched from a global counter, staged in
-//               shared memory (two buffers: the pair being retired and the next)
-//               and flattened into tiles; the contraction u_I += M f_J (and
-//               u_J += M f_I for J > I) is reduced per particle in shared memory
+// memory, 512 TMEM columns) and drive the tile engine of tc_mlp.cuh with two
+// streams of 128-evaluation tiles; a server warp per stream supplies the features of
+// the next tile while the engine runs the current one, and takes its outputs:
+//   k_near_tc : close pairs (I, J) fetched from a global counter by each stream,
+//               flattened into tiles; the contraction u_I += M f_J
+//               (and u_J += M f_I for J > I) is reduced per particle in shared memory
 //               and flushed with one FP64 atomic per particle and component per
 //               pair (src/CloseDot.cpp:245-299).
 //   k_far_tc  : column / row queries of all active ACA blocks, symmetrised into
@@ -30,286 +29,278 @@ __device__ __forceinline__ uint8_t* align1k(uint8_t* p) {
 constexpr int kTcLeaf = kTcMaxLeaf;
 
 struct NearStage {
-  float4 xI[kTcLeaf], xJ[kTcLeaf], fI[kTcLeaf], fJ[kTcLeaf];
   float uI[kTcLeaf][3], uJ[kTcLeaf][3];
 };
 
-// Three staging buffers: the pair of the tile being retired, of the tile in flight and of the
-// next tile can all differ (pairs of a single tile).
+// Velocity accumulators, two per stream: of the pair of the current tile and of the next one. (Positions and
+// forces are read through L1: the two leaves of a pair are at most 8 KB.)
 struct NearTcSmem {
   tc::Smem tcs;
-  NearStage st[3];
-  PairWork pw[3];
-  int item[3];
+  NearStage st[tc::kStreams][2];
 };
 static_assert(sizeof(NearTcSmem) + 1024 <= 232448, "near-field shared memory exceeds 227 KB per CTA");
 
-// u_I[i] += v for the rows of a warp: rows of a tile share few i (contiguous), so lanes with
-// equal i are summed by a segmented shuffle reduction and only segment heads add to shared memory.
-__device__ __forceinline__ void add_segmented(float (*uI)[3], int i, float v0, float v1, float v2) {
-  const unsigned act = __activemask();
-  if (act == 0xffffffffu) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float t0 = __shfl_down_sync(act, v0, o), t1 = __shfl_down_sync(act, v1, o),
-                  t2 = __shfl_down_sync(act, v2, o);
-      const int ko = __shfl_down_sync(act, i, o);
-      if (lane + o < 32 && ko == i) {
-        v0 += t0;
-        v1 += t1;
-        v2 += t2;
-      }
-    }
-    const int kp = __shfl_up_sync(act, i, 1);
-    if (lane == 0 || kp != i) {
-      atomicAdd(&uI[i][0], v0);
-      atomicAdd(&uI[i][1], v1);
-      atomicAdd(&uI[i][2], v2);
-    }
-  } else {
-    atomicAdd(&uI[i][0], v0);
-    atomicAdd(&uI[i][1], v1);
-    atomicAdd(&uI[i][2], v2);
-  }
-}
+constexpr int kParts = tc::kTile / 32;  // rows of a tile per server lane
 
-// Position of one 128-evaluation tile in the near-field stream and this thread's row of it.
+// A stream's position in the near-field work: tile [t0, t0 + 128) of a pair with accumulators buf, and
+// this lane's rows of it as (i, j). Consecutive tiles advance a row by 128 = di nJ + dj.
 struct NearTile {
-  int buf, t0;  // the pair itself is S.pw[buf]
-  int i, j;
-  bool valid, last;  // last: the final tile of its pair
-  float r[3];
+  PairWork pw;
+  int buf, t0, total, di, dj;
+  int i[kParts], j[kParts];
+  __device__ __forceinline__ bool last() const { return t0 + tc::kTile >= total; }
+  __device__ __forceinline__ bool valid(int k, int lane) const { return t0 + 32 * k + lane < total; }
 };
 
-// Next close pair from the global counter, staged into buffer b (all epilogue threads).
-__device__ __forceinline__ bool near_fetch(NearTcSmem& S, const NearArgs& a, int* counter, int b, NearTile& c) {
-  const int e = threadIdx.x;
-  // after an abort the stream ends here for every thread (the item is broadcast)
-  if (e == 0) S.item[b] = *(volatile int*)&S.tcs.abort_flag ? a.nwork : atomicAdd(counter, 1);
-  tc::epi_bar();  // also: every thread is done with the pair last staged in buffer b
-  const int item = S.item[b];
-  if (item >= a.nwork) return false;
+// The stream's next close pair (work item `item`) with cleared accumulators b; false at the end of the list.
+// `item` becomes the following item of the counter, drawn ahead of its use.
+__device__ __forceinline__ bool near_fetch(tc::Server& sv, NearStage& G, const NearArgs& a, int* counter, int b,
+                                           int& item, NearTile& c) {
+  const int lane = sv.lane;
+  if (item >= a.nwork || __any_sync(0xffffffffu, sv.aborted())) return false;
   const PairWork pw = a.work[item];
-  if (e == 0) S.pw[b] = pw;
-  NearStage& G = S.st[b];
-  for (int i = e; i < pw.nI; i += tc::kEpiThreads) {
-    G.xI[i] = a.xI[pw.sI + i];
-    G.fI[i] = a.fI[pw.sI + i];
-    G.uI[i][0] = G.uI[i][1] = G.uI[i][2] = 0.f;
-  }
-  for (int j = e; j < pw.nJ; j += tc::kEpiThreads) {
-    G.xJ[j] = a.xJ[pw.sJ + j];
-    G.fJ[j] = a.fJ[pw.sJ + j];
-    G.uJ[j][0] = G.uJ[j][1] = G.uJ[j][2] = 0.f;
-  }
-  tc::epi_bar();
+  if (lane == 0) item = gridDim.x + atomicAdd(counter, 1);
+  __syncwarp();  // every lane is done with the pair that last used accumulators b
+  for (int q = lane; q < 3 * pw.nI; q += 32) (&G.uI[0][0])[q] = 0.f;
+  for (int q = lane; q < 3 * pw.nJ; q += 32) (&G.uJ[0][0])[q] = 0.f;
+  item = __shfl_sync(0xffffffffu, item, 0);
+  c.pw = pw;
   c.buf = b;
   c.t0 = 0;
+  c.total = pw.nI * pw.nJ;
+  c.di = tc::kTile / pw.nJ;
+  c.dj = tc::kTile - c.di * pw.nJ;
+#pragma unroll
+  for (int k = 0; k < kParts; k++) {
+    c.i[k] = (32 * k + lane) / pw.nJ;
+    c.j[k] = 32 * k + lane - c.i[k] * pw.nJ;
+  }
+  __syncwarp();
   return true;
 }
 
-// This thread's row of a tile: (i, j) and the feature r = x_j - x_i (a dummy for padding rows).
-__device__ __forceinline__ void near_row(const NearTcSmem& S, NearTile& c, int row) {
-  const int nJ = S.pw[c.buf].nJ, total = S.pw[c.buf].nI * nJ;
-  const int flat = c.t0 + row;
-  c.valid = flat < total;
-  c.last = c.t0 + tc::kTile >= total;
-  c.i = c.valid ? flat / nJ : 0;
-  c.j = c.valid ? flat - c.i * nJ : 0;
-  c.r[0] = 1.f;
-  c.r[1] = c.r[2] = 0.f;
-  if (c.valid) {
-    const float4 xi = S.st[c.buf].xI[c.i], xj = S.st[c.buf].xJ[c.j];
-    c.r[0] = xj.x - xi.x;
-    c.r[1] = xj.y - xi.y;
-    c.r[2] = xj.z - xi.z;
+__device__ __forceinline__ void near_advance(NearTile& c) {
+  c.t0 += tc::kTile;
+#pragma unroll
+  for (int k = 0; k < kParts; k++) {
+    c.i[k] += c.di;
+    c.j[k] += c.dj;
+    if (c.j[k] >= c.pw.nJ) {
+      c.j[k] -= c.pw.nJ;
+      c.i[k]++;
+    }
   }
 }
 
-// Contraction of one retired tile: u_I += M f_J (part 0), u_J += M f_I for J > I (part 1)
-// (src/CloseDot.cpp:245-299), into the pair's shared-memory accumulators.
-__device__ __forceinline__ void near_use(NearTcSmem& S, const NearTile& c, int p, float (&M)[9]) {
-  if (!c.valid || p >= 2) return;
-  NearStage& G = S.st[c.buf];
-  const int flags = S.pw[c.buf].flags;
-  if (flags & kPairSymmetrize) {
+// Features r = x_j - x_i of tile t (a dummy for padding rows).
+__device__ __forceinline__ void near_put(tc::Server& sv, const NearArgs& a, const NearTile& c, uint32_t t) {
 #pragma unroll
-    for (int q = 0; q < 3; q++)
+  for (int k = 0; k < kParts; k++) {
+    float r[3] = {1.f, 0.f, 0.f};
+    if (c.valid(k, sv.lane)) {
+      const float4 xi = __ldg(&a.xI[c.pw.sI + c.i[k]]), xj = __ldg(&a.xJ[c.pw.sJ + c.j[k]]);
+      r[0] = xj.x - xi.x;
+      r[1] = xj.y - xi.y;
+      r[2] = xj.z - xi.z;
+    }
+    sv.put(t, 32 * k + sv.lane, r[0], r[1], r[2]);
+  }
+  sv.ready();
+}
+
+// Contraction of tile t into the pair's shared-memory accumulators: u_I += M f_J and for J > I
+// u_J += M f_I (the same M, not transposed; src/CloseDot.cpp:245-299). One warp owns the stream's
+// accumulators. The rows of a part are consecutive in j, so its lanes hold distinct j when nJ >= 32.
+__device__ __forceinline__ void near_take(tc::Server& sv, NearStage& G, const NearArgs& a, const NearTile& c, uint32_t t) {
+  float v[kParts][3];
+  const bool distinct = c.pw.nJ >= 32;
 #pragma unroll
-      for (int k = q + 1; k < 3; k++) {
-        const float v = 0.5f * (M[3 * q + k] + M[3 * k + q]);
-        M[3 * q + k] = v;
-        M[3 * k + q] = v;
+  for (int k = 0; k < kParts; k++) {
+    v[k][0] = v[k][1] = v[k][2] = 0.f;
+    if (c.valid(k, sv.lane)) {
+      float M[9];
+      sv.take(t, 32 * k + sv.lane, M);
+      const float4 fj = __ldg(&a.fJ[c.pw.sJ + c.j[k]]);
+#pragma unroll
+      for (int q = 0; q < 3; q++) v[k][q] = M[3 * q] * fj.x + M[3 * q + 1] * fj.y + M[3 * q + 2] * fj.z;
+      if (c.pw.flags & kPairTransposed) {
+        const float4 fi = __ldg(&a.fI[c.pw.sI + c.i[k]]);
+        float* u = G.uJ[c.j[k]];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+          const float w = M[3 * q] * fi.x + M[3 * q + 1] * fi.y + M[3 * q + 2] * fi.z;
+          if (distinct)
+            u[q] += w;
+          else
+            atomicAdd(&u[q], w);
+        }
       }
+    }
+    __syncwarp();  // the next part's lanes may hold the same j
   }
-  if (p == 0) {
-    const float4 fj = G.fJ[c.j];
-    add_segmented(G.uI, c.i, M[0] * fj.x + M[1] * fj.y + M[2] * fj.z, M[3] * fj.x + M[4] * fj.y + M[5] * fj.z,
-                  M[6] * fj.x + M[7] * fj.y + M[8] * fj.z);
-  } else if (flags & kPairTransposed) {  // same M, not transposed (src/CloseDot.cpp:281-298)
-    const float4 fi = G.fI[c.i];
-    atomicAdd(&G.uJ[c.j][0], M[0] * fi.x + M[1] * fi.y + M[2] * fi.z);
-    atomicAdd(&G.uJ[c.j][1], M[3] * fi.x + M[4] * fi.y + M[5] * fi.z);
-    atomicAdd(&G.uJ[c.j][2], M[6] * fi.x + M[7] * fi.y + M[8] * fi.z);
+  // u_I: the tile's rows cover the targets i0 .. i1; each one's rows are summed over lanes
+  const int i0 = c.t0 / c.pw.nJ;
+  const int tail = min(c.t0 + tc::kTile, c.total) - 1, i1 = tail / c.pw.nJ;
+  for (int i = i0; i <= i1; i++) {
+    float w[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < kParts; k++)
+      if (c.i[k] == i)
+#pragma unroll
+        for (int q = 0; q < 3; q++) w[q] += v[k][q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < 3; q++) w[q] += __shfl_xor_sync(0xffffffffu, w[q], o);
+    if (sv.lane < 3) G.uI[i][sv.lane] += sv.lane == 0 ? w[0] : sv.lane == 1 ? w[1] : w[2];
   }
 }
 
-// The pair of a retired last tile is complete: flush its velocities (all epilogue threads).
-__device__ __forceinline__ void near_flush(NearTcSmem& S, const NearArgs& a, const NearTile& c) {
-  tc::epi_bar();
-  if (*(volatile int*)&S.tcs.abort_flag) return;  // the launch reports an error; nothing is added
-  const NearStage& G = S.st[c.buf];
-  const PairWork pw = S.pw[c.buf];
-  for (int q = threadIdx.x; q < 3 * pw.nI; q += tc::kEpiThreads)
-    atomicAdd(&a.uI[3 * (size_t)pw.sI + q], (double)(&G.uI[0][0])[q]);
+// A finished pair's velocities: one FP64 atomic per particle and component.
+__device__ __forceinline__ void near_flush(const tc::Server& sv, const NearStage& G, const NearArgs& a,
+                                           const PairWork& pw) {
+  __syncwarp();
+  for (int q = sv.lane; q < 3 * pw.nI; q += 32) atomicAdd(&a.uI[3 * (size_t)pw.sI + q], (double)(&G.uI[0][0])[q]);
   if (pw.flags & kPairTransposed)
-    for (int q = threadIdx.x; q < 3 * pw.nJ; q += tc::kEpiThreads)
-      atomicAdd(&a.uJ[3 * (size_t)pw.sJ + q], (double)(&G.uJ[0][0])[q]);
+    for (int q = sv.lane; q < 3 * pw.nJ; q += 32) atomicAdd(&a.uJ[3 * (size_t)pw.sJ + q], (double)(&G.uJ[0][0])[q]);
 }
 
 __global__ void __launch_bounds__(tc::kThreads, 1)
     k_near_tc(NearArgs a, TcWeights w, int* work_counter, int* err) {
   extern __shared__ uint8_t smem_raw[];
   NearTcSmem& S = *reinterpret_cast<NearTcSmem*>(align1k(smem_raw));
-  tc::cta_setup(S.tcs, w);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == tc::kMmaWarp) {
-    if (lane == 0) tc::mma_loop(S.tcs, err);
-    __syncwarp();
-  } else {
-    const long long t_start = clock64();
-    const int row = tc::epi_row(), p = tc::epi_part();
-    tc::Epi eng{S.tcs, err, S.tcs.tmem_base + ((uint32_t)(32 * ((threadIdx.x >> 5) & 3)) << 16), p};
-    NearTile prev{}, cur{};
-    int nbuf = 0;  // staging buffers are used in turn
-    const bool have = near_fetch(S, a, work_counter, nbuf, cur);
-    nbuf = (nbuf + 1) % 3;
-    if (have) near_row(S, cur, row);
-    eng.start(have, cur.r[0], cur.r[1], cur.r[2]);
-    bool has_prev = false;
-    // The control flow is uniform over the epilogue threads (tile positions and work items are
-    // shared), so the named barriers of near_fetch / near_flush are always reached by all of them;
-    // after an abort the engine calls return at once and near_fetch ends the stream.
-    while (have) {
-      // the next tile: the rest of this pair, or the next pair staged into the next buffer
+  tc::run_cta(S.tcs, w, err, [&](tc::Server sv) {
+    NearStage* G = S.st[sv.stream];
+    // stream 0 of every CTA starts with the item of its block index, the rest come from the counter
+    int item = blockIdx.x;
+    if (sv.stream != 0) {
+      if (sv.lane == 0) item = gridDim.x + atomicAdd(work_counter, 1);
+      item = __shfl_sync(0xffffffffu, item, 0);
+    }
+    NearTile cur{};
+    bool have = near_fetch(sv, G[0], a, work_counter, 0, item, cur);
+    if (have)
+      near_put(sv, a, cur, 0);
+    else
+      sv.end(0);
+    for (uint32_t t = 0; have; t++) {
+      // the next tile: the rest of this pair, or the next pair with the other accumulators
       NearTile nxt = cur;
-      nxt.t0 += tc::kTile;
       bool has_next = true;
-      if (cur.last) {
-        has_next = near_fetch(S, a, work_counter, nbuf, nxt);
-        nbuf = (nbuf + 1) % 3;
-      }
-      if (has_next) near_row(S, nxt, row);
-      eng.step(has_next, nxt.r[0], nxt.r[1], nxt.r[2], prev.r[0], prev.r[1], prev.r[2],
-               [&](float (&M)[9]) { near_use(S, prev, p, M); });
-      if (has_prev && prev.last) near_flush(S, a, prev);
-      prev = cur;
-      has_prev = true;
-      if (!has_next) break;
+      if (cur.last())
+        has_next = near_fetch(sv, G[cur.buf ^ 1], a, work_counter, cur.buf ^ 1, item, nxt);
+      else
+        near_advance(nxt);
+      if (has_next)
+        near_put(sv, a, nxt, t + 1);
+      else
+        sv.end(t + 1);
+      if (!sv.wait(t)) return;  // the launch reports an error
+      near_take(sv, G[cur.buf], a, cur, t);
+      if (cur.last()) near_flush(sv, G[cur.buf], a, cur.pw);
       cur = nxt;
+      have = has_next;
     }
-    if (has_prev) {
-      eng.finish(prev.r[0], prev.r[1], prev.r[2], [&](float (&M)[9]) { near_use(S, prev, p, M); });
-      near_flush(S, a, prev);
-    }
-    if (S.tcs.prof && threadIdx.x == 0) S.tcs.wprof[12] += (unsigned long long)(clock64() - t_start);
-  }
-  tc::cta_teardown(S.tcs);
+  });
 }
 
 struct FarTcSmem {
   tc::Smem tcs;
 };
 
-// This thread's row of far tile `tile`: block b, local index loc, term k, feature r.
-struct FarRow {
-  int b, loc, k;
-  bool valid;
-  float r[3];
+// This lane's rows of a far tile: their entries in the C / Q pool (-1: none).
+struct FarTile {
+  long long dst[kParts];
 };
 
-__device__ __forceinline__ void far_row(const FarArgs& a, int which, int nact, int tot, int tile, int row, FarRow& f) {
-  const int g = tile * tc::kTile + row;
-  f.r[0] = 1.f;
-  f.r[1] = f.r[2] = 0.f;
-  f.valid = g < tot;
-  if (!f.valid) return;
+__device__ __forceinline__ void far_put(tc::Server& sv, const FarArgs& a, int which, int nact, int tot, int tile,
+                                        uint32_t t, FarTile& c) {
   const int32_t* pre = which ? a.preJ : a.preI;
-  int lo = 0, hi = nact;
+  // the block of the tile's first row: 32-way search of the active blocks' prefix
+  const int g0 = tile * tc::kTile;
+  int lo = 0, hi = nact;  // pre[lo] <= g0 < pre[hi]
   while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (pre[mid] <= g)
-      lo = mid;
-    else
-      hi = mid;
+    const int step = (hi - lo + 31) / 32, p = lo + sv.lane * step;
+    const unsigned m = __ballot_sync(0xffffffffu, sv.lane > 0 && p < hi && pre[p] <= g0);
+    lo += __popc(m) * step;
+    hi = min(hi, lo + step);
   }
-  f.b = a.act[lo];
-  f.loc = g - pre[lo];
-  const FarBlock bk = a.blocks[f.b];
-  f.k = a.state[f.b].k;
-  float4 xi, xj;
-  if (which == 0) {
-    xj = a.x[bk.sJ + a.cols[(size_t)f.b * a.ldr + f.k]];
-    xi = a.x[bk.sI + f.loc];
-  } else {
-    xj = a.x[bk.sJ + f.loc];
-    xi = a.x[bk.sI + a.rows[(size_t)f.b * a.ldr + f.k]];
-  }
-  f.r[0] = xj.x - xi.x;
-  f.r[1] = xj.y - xi.y;
-  f.r[2] = xj.z - xi.z;
-}
-
-// symmetrised 3x3 of a retired far row into the C (which = 0) or Q pool; the two threads of a
-// row store alternate entries (src/FarDot.cpp:445-456: diagonal copied, off-diagonal halved sum)
-__device__ __forceinline__ void far_use(const FarArgs& a, int which, const FarRow& f, int p, const float (&M)[9]) {
-  if (!f.valid || p >= 2) return;
-  const FarBlock bk = a.blocks[f.b];
-  pool_t* dst = which == 0 ? a.C + 9 * (bk.cOff + (int64_t)f.k * bk.nI + f.loc)
-                           : a.Q + 9 * (bk.qOff + (int64_t)f.k * bk.nJ + f.loc);
 #pragma unroll
-  for (int q = 0; q < 9; q++) {
-    if ((q & 1) != p) continue;
-    const int rr = q / 3, c = q % 3;
-    dst[q] = (rr == c) ? M[q] : 0.5f * (M[3 * rr + c] + M[3 * c + rr]);  // the FP32 half-sum is exact in FP64 too
+  for (int k = 0; k < kParts; k++) {
+    const int g = g0 + 32 * k + sv.lane;
+    float r[3] = {1.f, 0.f, 0.f};
+    c.dst[k] = -1;
+    if (g < tot) {
+      while (pre[lo + 1] <= g) lo++;
+      const int b = a.act[lo], loc = g - pre[lo];
+      const FarBlock bk = a.blocks[b];
+      const int it = a.state[b].k;
+      float4 xi, xj;
+      if (which == 0) {
+        xj = a.x[bk.sJ + a.cols[(size_t)b * a.ldr + it]];
+        xi = a.x[bk.sI + loc];
+        c.dst[k] = bk.cOff + (int64_t)it * bk.nI + loc;
+      } else {
+        xj = a.x[bk.sJ + loc];
+        xi = a.x[bk.sI + a.rows[(size_t)b * a.ldr + it]];
+        c.dst[k] = bk.qOff + (int64_t)it * bk.nJ + loc;
+      }
+      r[0] = xj.x - xi.x;
+      r[1] = xj.y - xi.y;
+      r[2] = xj.z - xi.z;
+    }
+    sv.put(t, 32 * k + sv.lane, r[0], r[1], r[2]);
   }
+  sv.ready();
 }
 
-__global__ void __launch_bounds__(tc::kThreads, 1) k_far_tc(FarArgs a, TcWeights w, int which, int* err) {
+// symmetrised 3x3 of each row into the C / Q pool (src/FarDot.cpp:445-456: diagonal copied,
+// off-diagonal halved sum)
+__device__ __forceinline__ void far_take(tc::Server& sv, pool_t* pool, const FarTile& c, uint32_t t) {
+#pragma unroll
+  for (int k = 0; k < kParts; k++)
+    if (c.dst[k] >= 0) {
+      float M[9];
+      sv.take(t, 32 * k + sv.lane, M);
+      pool_t* dst = pool + 9 * c.dst[k];
+#pragma unroll
+      for (int q = 0; q < 9; q++) {
+        const int rr = q / 3, cc = q % 3;
+        dst[q] = rr == cc ? M[q] : 0.5f * __fadd_rn(M[3 * rr + cc], M[3 * cc + rr]);  // the FP32 half-sum is exact in FP64 too
+      }
+    }
+}
+
+__global__ void __launch_bounds__(tc::kThreads, 1)
+    k_far_tc(FarArgs a, TcWeights w, int which, int* err) {
   extern __shared__ uint8_t smem_raw[];
   FarTcSmem& S = *reinterpret_cast<FarTcSmem*>(align1k(smem_raw));
   const int nact = a.ctr[kCtrActive];
   const int tot = which ? a.ctr[kCtrTotJ] : a.ctr[kCtrTotI];
   if ((int)blockIdx.x * tc::kTile >= tot) return;  // uniform: before any setup
-  tc::cta_setup(S.tcs, w);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == tc::kMmaWarp) {
-    if (lane == 0) tc::mma_loop(S.tcs, err);
-    __syncwarp();
-  } else {
-    const int row = tc::epi_row(), p = tc::epi_part();
-    tc::Epi eng{S.tcs, err, S.tcs.tmem_base + ((uint32_t)(32 * ((threadIdx.x >> 5) & 3)) << 16), p};
-    int tile = blockIdx.x;
-    FarRow prev{}, cur{};
-    far_row(a, which, nact, tot, tile, row, cur);
-    eng.start(true, cur.r[0], cur.r[1], cur.r[2]);
-    for (;;) {  // uniform over the epilogue threads; after an abort the engine calls return at once
-      const int nt = tile + gridDim.x;
-      const bool has_next = nt * tc::kTile < tot;
-      FarRow nxt{};
-      nxt.r[0] = 1.f;
-      if (has_next) far_row(a, which, nact, tot, nt, row, nxt);
-      eng.step(has_next, nxt.r[0], nxt.r[1], nxt.r[2], prev.r[0], prev.r[1], prev.r[2],
-               [&](float (&M)[9]) { far_use(a, which, prev, p, M); });
-      prev = cur;
-      if (!has_next) break;
-      tile = nt;
+  tc::run_cta(S.tcs, w, err, [&](tc::Server sv) {
+    pool_t* pool = which ? a.Q : a.C;
+    int tile = blockIdx.x + gridDim.x * sv.stream;
+    FarTile cur{};
+    bool have = tile * tc::kTile < tot;
+    if (have)
+      far_put(sv, a, which, nact, tot, tile, 0, cur);
+    else
+      sv.end(0);
+    for (uint32_t t = 0; have; t++) {
+      tile += tc::kStreams * gridDim.x;
+      const bool has_next = tile * tc::kTile < tot;
+      FarTile nxt{};
+      if (has_next)
+        far_put(sv, a, which, nact, tot, tile, t + 1, nxt);
+      else
+        sv.end(t + 1);
+      if (!sv.wait(t)) return;
+      far_take(sv, pool, cur, t);
       cur = nxt;
+      have = has_next;
     }
-    eng.finish(prev.r[0], prev.r[1], prev.r[2], [&](float (&M)[9]) { far_use(a, which, prev, p, M); });
-  }
-  tc::cta_teardown(S.tcs);
+  });
   if (threadIdx.x == 0 && blockIdx.x == 0) atomicAdd(a.evals, (unsigned long long)tot);
 }
 
@@ -317,61 +308,48 @@ struct EvalTcSmem {
   tc::Smem tcs;
 };
 
-struct EvalRow {
-  int64_t g;
-  bool valid;
-  float r[3];
-};
-
-__device__ __forceinline__ void eval_row(const float* __restrict__ r, int64_t n, int64_t tile, int row, EvalRow& f) {
-  f.g = tile * tc::kTile + row;
-  f.valid = f.g < n;
-  f.r[0] = 1.f;
-  f.r[1] = f.r[2] = 0.f;
-  if (!f.valid) return;
-  f.r[0] = r[3 * f.g];
-  f.r[1] = r[3 * f.g + 1];
-  f.r[2] = r[3 * f.g + 2];
-}
-
 __global__ void __launch_bounds__(tc::kThreads, 1)
     k_eval_tc(const float* __restrict__ r, float* __restrict__ y, int64_t n, TcWeights w, int* err) {
   extern __shared__ uint8_t smem_raw[];
   EvalTcSmem& S = *reinterpret_cast<EvalTcSmem*>(align1k(smem_raw));
-  tc::cta_setup(S.tcs, w);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == tc::kMmaWarp) {
-    if (lane == 0) tc::mma_loop(S.tcs, err);
-    __syncwarp();
-  } else {
-    const int row = tc::epi_row(), p = tc::epi_part();
-    tc::Epi eng{S.tcs, err, S.tcs.tmem_base + ((uint32_t)(32 * ((threadIdx.x >> 5) & 3)) << 16), p};
-    auto use = [&](const EvalRow& f, float(&M)[9]) {
-      if (f.valid && p < 2)  // the two threads of a row store alternate entries
+  tc::run_cta(S.tcs, w, err, [&](tc::Server sv) {
+    auto put = [&](int64_t tile, uint32_t t) {
 #pragma unroll
-        for (int q = 0; q < 9; q++)
-          if ((q & 1) == p) y[9 * f.g + q] = M[q];
+      for (int k = 0; k < kParts; k++) {
+        const int64_t g = tile * tc::kTile + 32 * k + sv.lane;
+        const bool in = g < n;
+        sv.put(t, 32 * k + sv.lane, in ? r[3 * g] : 1.f, in ? r[3 * g + 1] : 0.f, in ? r[3 * g + 2] : 0.f);
+      }
+      sv.ready();
     };
-    int64_t tile = blockIdx.x;
-    EvalRow prev{}, cur{};
-    eval_row(r, n, tile, row, cur);
-    eng.start(true, cur.r[0], cur.r[1], cur.r[2]);
-    for (;;) {  // uniform over the epilogue threads; after an abort the engine calls return at once
-      const int64_t nt = tile + gridDim.x;
+    int64_t tile = blockIdx.x + (int64_t)gridDim.x * sv.stream;
+    bool have = tile * tc::kTile < n;
+    if (have)
+      put(tile, 0);
+    else
+      sv.end(0);
+    for (uint32_t t = 0; have; t++) {
+      const int64_t nt = tile + tc::kStreams * (int64_t)gridDim.x;
       const bool has_next = nt * tc::kTile < n;
-      EvalRow nxt{};
-      nxt.r[0] = 1.f;
-      if (has_next) eval_row(r, n, nt, row, nxt);
-      eng.step(has_next, nxt.r[0], nxt.r[1], nxt.r[2], prev.r[0], prev.r[1], prev.r[2],
-               [&](float (&M)[9]) { use(prev, M); });
-      prev = cur;
-      if (!has_next) break;
-      tile = nt;
-      cur = nxt;
+      if (has_next)
+        put(nt, t + 1);
+      else
+        sv.end(t + 1);
+      if (!sv.wait(t)) return;
+#pragma unroll
+      for (int k = 0; k < kParts; k++) {
+        const int64_t g = tile * tc::kTile + 32 * k + sv.lane;
+        if (g < n) {
+          float M[9];
+          sv.take(t, 32 * k + sv.lane, M);
+#pragma unroll
+          for (int q = 0; q < 9; q++) y[9 * g + q] = M[q];
+        }
+      }
+          tile = nt;
+      have = has_next;
     }
-    eng.finish(prev.r[0], prev.r[1], prev.r[2], [&](float (&M)[9]) { use(prev, M); });
-  }
-  tc::cta_teardown(S.tcs);
+  });
 }
 
 template <class K>
