@@ -116,6 +116,7 @@ struct hignn_model {
   hignn::BlockLists lists;
   std::vector<float> xt;   // tree order
   std::vector<int64_t> inv_perm;
+  std::vector<int64_t> close_item0;  // first near-field work item of each close pair (size num_close + 1)
   bool tree_ready = false;
   bool lists_sym = true;
   int64_t lists_max_rel = 500000;
@@ -199,6 +200,8 @@ void require_device(hignn_model* m) {
   if (m->device < 0) throw Error(HIGNN_ERR_NODEV, "model was created without a CUDA device (host-only)");
   HIGNN_CUDA(cudaSetDevice(m->device));
 }
+
+constexpr int64_t kItemEvals = 128;  // near-field work items are cut at multiples of a tile
 
 // Builds the tree and lists of m->xyz and, on a device model, uploads the tree-order positions
 // and the close work list. Everything is built and checked before the model changes: a tree that
@@ -300,10 +303,23 @@ void build_structures(hignn_model* m) {
     perm[i] = (int32_t)m->tree.perm[i];
     slot[i] = (int32_t)m->inv_perm[i];
   }
-  // close work list (src/CloseFarCheck.cpp:298-336 order)
-  std::vector<hignn::PairWork> work(m->lists.closeI.size());
+  // close work list (src/CloseFarCheck.cpp:298-336 order). Where the pairs are too few to keep every SM
+  // busy to the end (two work items in flight per SM, about eight per slot wanted), they are cut into
+  // runs of evaluations, whole tiles each; m->close_item0 gives every pair's first item. (601 spheres have 109
+  // pairs for 148 SMs; their plain product took 3.65 ms with whole pairs, 2.03 ms with both this and the
+  // faster network; from about 100,000 particles on no pair is cut.)
+  std::vector<hignn::PairWork> work;
+  const size_t nclose = m->lists.closeI.size();
+  work.reserve(nclose);
   int64_t evals = 0;
-  for (size_t q = 0; q < work.size(); q++) {
+  for (size_t q = 0; q < nclose; q++) {
+    const auto& I = m->tree.nodes[m->lists.closeI[q]];
+    const auto& J = m->tree.nodes[m->lists.closeJ[q]];
+    evals += (I.end - I.start) * (J.end - J.start);
+  }
+  const int64_t per_item = (evals / (8 * 2 * (int64_t)std::max(1, m->num_sms)) / kItemEvals + 1) * kItemEvals;
+  m->close_item0.resize(nclose + 1);
+  for (size_t q = 0; q < nclose; q++) {
     const auto& I = m->tree.nodes[m->lists.closeI[q]];
     const auto& J = m->tree.nodes[m->lists.closeJ[q]];
     hignn::PairWork w{};
@@ -312,9 +328,15 @@ void build_structures(hignn_model* m) {
     w.sJ = (int32_t)J.start;
     w.nJ = (int32_t)(J.end - J.start);
     w.flags = (m->use_symmetry && m->lists.closeJ[q] > m->lists.closeI[q]) ? hignn::kPairTransposed : 0;
-    evals += (int64_t)w.nI * w.nJ;
-    work[q] = w;
+    m->close_item0[q] = (int64_t)work.size();
+    const int64_t total = (int64_t)w.nI * w.nJ;
+    for (int64_t e = 0; e < total; e += per_item) {
+      w.first = (int32_t)e;
+      w.count = (int32_t)std::min(per_item, total - e);
+      work.push_back(w);
+    }
   }
+  m->close_item0[nclose] = (int64_t)work.size();
   m->stats.close_evals = evals;
   m->max_leaf = 0;
   for (const auto& w : work) m->max_leaf = std::max(m->max_leaf, std::max(w.nI, w.nJ));
@@ -808,8 +830,9 @@ void far_field(hignn_model* m) {
 void near_field(hignn_model* m) {
   hignn::NearArgs a{};
   ensure_shard(m);
-  a.work = m->close_work.as<hignn::PairWork>() + m->sh_c0;
-  a.nwork = (int)(m->sh_c1 - m->sh_c0);
+  const int64_t i0 = m->close_item0[m->sh_c0], i1 = m->close_item0[m->sh_c1];
+  a.work = m->close_work.as<hignn::PairWork>() + i0;
+  a.nwork = (int)(i1 - i0);
   a.xI = a.xJ = m->x4.as<float4>();
   a.fI = a.fJ = m->f4.as<float4>();
   a.uI = a.uJ = m->u.as<double>();
@@ -919,8 +942,8 @@ uint64_t graph_signature(hignn_model* m) {
   mix((uint64_t)m->max_iter);
   mix((uint64_t)m->use_symmetry);
   mix((uint64_t)m->has_student);
-  mix((uint64_t)m->sh_c0);
-  mix((uint64_t)m->sh_c1);
+  mix((uint64_t)m->close_item0[m->sh_c0]);
+  mix((uint64_t)m->close_item0[m->sh_c1]);
   mix((uint64_t)m->batches.size());
   for (const auto& bt : m->batches) mix(((uint64_t)bt.b0 << 40) ^ ((uint64_t)bt.b1 << 16) ^ (uint64_t)bt.iters);
   uint64_t e, t;

@@ -94,11 +94,13 @@ struct TcWeights {
   unsigned long long* prof = nullptr;  // optional wait profile of the engine (tc::kProfSlots counters)
 };
 
-// One unit of near-field (or dense) work: target range I against source range J.
+// One unit of near-field (or dense) work: target range I against source range J, or of its
+// evaluations i nJ + j only those from `first` on, `count` of them (count 0: the whole pair).
 constexpr int32_t kPairTransposed = 1;  // also u_J += M f_I (symmetric close pair, J > I)
 constexpr int32_t kPairSymmetrize = 2;  // use 0.5 (M + M^T) (dense product)
 struct PairWork {
-  int32_t sI, nI, sJ, nJ, flags, pad0, pad1, pad2;
+  int32_t sI, nI, sJ, nJ, flags, first, count, pad;
 };
+__host__ __device__ inline int pair_end(const PairWork& w) { return w.count ? w.first + w.count : w.nI * w.nJ; }
 
 }  // namespace hignn

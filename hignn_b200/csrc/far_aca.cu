@@ -235,8 +235,9 @@ struct EvalSmem {
   int32_t loc[simt::kTile];
 };
 
-// Column (which = 0) or row (which = 1) queries of every active block, 128 per tile.
-__global__ void __launch_bounds__(simt::kThreads, 1) k_far_eval(FarArgs a, MlpF32 w, int which) {
+// Column (which = 0) or row (which = 1) queries of every active block, one tile of simt::kTile per CTA at a time.
+__global__ void __launch_bounds__(simt::kThreads, simt::kCtasPerSm)
+    k_far_eval(FarArgs a, MlpF32 w, int which) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   EvalSmem& s = *reinterpret_cast<EvalSmem*>(smem_raw);
   const int t = threadIdx.x;
@@ -1028,7 +1029,7 @@ void far_iteration(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, cons
   else if (tcw)
     launch_far_tc(a, *tcw, 0, err, num_sms, s);
   else
-    k_far_eval<<<num_sms, simt::kThreads, eval_smem, s>>>(a, w, 0);
+    k_far_eval<<<simt::kCtasPerSm * num_sms, simt::kThreads, eval_smem, s>>>(a, w, 0);
   mark();
   if (a.fast_pivots)
     k_far_col_pivot_f32<<<piv_grid, kPivThreads, col_smem_f32(a.ldr), s>>>(a);
@@ -1040,7 +1041,7 @@ void far_iteration(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, cons
   else if (tcw)
     launch_far_tc(a, *tcw, 1, err, num_sms, s);
   else
-    k_far_eval<<<num_sms, simt::kThreads, eval_smem, s>>>(a, w, 1);
+    k_far_eval<<<simt::kCtasPerSm * num_sms, simt::kThreads, eval_smem, s>>>(a, w, 1);
   mark();
   if (a.fast_pivots)
     k_far_row_pivot_f32<<<piv_grid, kPivThreads, row_smem_f32(a.ldr), s>>>(a);

@@ -41,7 +41,7 @@ __global__ void k_gather_positions(const float4* __restrict__ x4, const int32_t*
   out[i] = x4[pos[i]];
 }
 
-__global__ void __launch_bounds__(simt::kThreads, 1)
+__global__ void __launch_bounds__(simt::kThreads, simt::kCtasPerSm)
     k_eval_simt(const float* __restrict__ r, float* __restrict__ y, int64_t n, MlpF32 w) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   simt::Smem& s = *reinterpret_cast<simt::Smem*>(smem_raw);
@@ -85,7 +85,7 @@ void launch_eval_simt(const float* r, float* y, int64_t n, const MlpF32& w, int 
   const size_t smem = sizeof(simt::Smem);
   HIGNN_CUDA(cudaFuncSetAttribute(k_eval_simt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int64_t tiles = (n + simt::kTile - 1) / simt::kTile;
-  int grid = (int)(tiles < num_sms ? tiles : num_sms);
+  int grid = (int)(tiles < simt::kCtasPerSm * num_sms ? tiles : simt::kCtasPerSm * num_sms);
   k_eval_simt<<<grid, simt::kThreads, smem, s>>>(r, y, n, w);
   HIGNN_CHECK_LAUNCH();
 }

@@ -1,4 +1,4 @@
-// FP32 SIMT evaluation of the two-body network, 128 evaluations per tile.
+// FP32 SIMT evaluation of the two-body network, 64 evaluations per tile.
 //
 // This is the "plain FP32" form: every layer in FP32 on the CUDA cores, the same
 // arithmetic class as the reference's libtorch FP32 forward (src/CloseDot.cpp:233).
@@ -10,36 +10,52 @@
 //   y[o]  = (sum_n fma(h2[n], W3[o][n], .), n ascending from 0) + b3[o] (+ 1 on the
 //           diagonal), divided by |r| = sqrt(fma(r_z, r_z, fma(r_y, r_y, r_x r_x))).
 //
-// Tile schedule (256 threads): layer 1 fills h1[k][e]; layer 2 runs in 8
-// chunks of 64 hidden units, each a 128x64x128 register-tiled GEMM (8 evals x
-// 4 units per thread) on W2 chunks double-buffered in shared memory with
-// cp.async; each chunk is tanh'd into h2[n][e] and immediately folded into
-// the 9 layer-3 outputs, so the 512-wide activation never leaves the SM.
+// The bound is the FP32 pipe: 70,528 FMA per evaluation (551 clocks per SM) and 640 tanh of about 24
+// FMA-pipe slots each. Two CTAs of four warps share an SM, so that one's tanh and layer 3 run under
+// the other's layer 2. A warp owns 16 evaluations from features to outputs; only the W2 slices are shared:
+//   layer 2 in two chunks of 256 units, 16 evaluations x 8 units per thread as packed FMAs (fma.rn.f32x2
+//   over evaluation pairs: half the issue slots, the same rounding); per k a thread reads
+//   16 h1 values (broadcast) and 8 weights, 24 clocks of shared-memory return for 128 of the
+//   warp's FMA pipe; W2 comes in slices of 8 k x 256 units, double-buffered with cp.async;
+//   each chunk's sums go through tanh and layer 3 in four pieces of 64 units by way of 5 KB of the
+//   warp's shared memory; in layer 3 a lane takes two evaluations and three outputs (W3 read through the
+//   constant bank instead was four times slower: its loads do not pipeline).
+// Measured (one B200, 1.0M separations): 2.22e8 evaluations/s, against 1.54e8 of one CTA of eight warps per SM
+// with 8 x 4 scalar FMAs per thread, branching tanh and one weight read per FMA in layer 3. Layer 2 alone
+// runs at 3.4e8 (62 % of the FP32 pipe; the packed FMA itself reaches 77 % of it with two warps per
+// sub-partition, and scalar FMAs in the same tile are 5 % slower), layer 2 and tanh at 2.4e8.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include "common.h"
 #include "tanh_f32.cuh"
+#include "tanh_f32x2.cuh"
 
 namespace hignn {
 namespace simt {
 
-constexpr int kThreads = 256;
-constexpr int kTile = 128;
-constexpr int kChunk = 64;
-constexpr int kNumChunks = kH2 / kChunk;
+constexpr int kWarps = 4;
+constexpr int kThreads = 32 * kWarps;
+constexpr int kRows = 16;               // evaluations per warp
+constexpr int kTile = kRows * kWarps;   // per CTA
+constexpr int kCtasPerSm = 2;
+constexpr int kChunk = 256;             // layer-2 units per pass over k
+constexpr int kSlice = 8;               // k per staged W2 slice
+constexpr int kSlices = kH1 / kSlice;
+constexpr int kPiece = 64;              // units per tanh / layer-3 piece
+constexpr int kPieceStride = kRows + 4; // floats per unit: 16-byte stores of consecutive units hit 32 banks
 
 struct Smem {
-  float h1[kH1][kTile];           // 64 KB, [k][e]
-  float w2[2][kH1][kChunk];       // 64 KB, W2^T chunks [k][n]
-  float h2[kChunk][kTile];        // 32 KB, [n][e]
-  float w3[kOut][kH2];            // 18 KB
-  float b2[kH2];                  // 2 KB
-  float4 w1b1[kH1];               // 2 KB
+  float h1[kH1][kTile];                          // 32 KB, [k][e]
+  float w2[2][kSlice][kChunk];                   // 16 KB, W2^T slices [k][n]
+  float h2[kWarps][kPiece][kPieceStride];        // 20 KB, [n][e] of each warp
+  float w3[kOut][kH2];                           // 18 KB
+  float b2[kH2];                                 // 2 KB
+  float4 w1b1[kH1];                              // 2 KB
   float b3[16];
-  float4 r[kTile];                // features (x, y, z, unused)
-  float y[kTile][kOut + 1];       // network outputs after the wrapper
+  float4 r[kTile];                               // features (x, y, z, unused)
+  float y[kTile][kOut + 1];                      // network outputs after the wrapper
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -52,98 +68,129 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // Per-CTA weight staging (once per kernel).
 __device__ __forceinline__ void load_weights(Smem& s, const MlpF32& w) {
   const int t = threadIdx.x;
-  for (int i = t; i < kOut * kH2; i += kThreads) (&s.w3[0][0])[i] = w.w3[i];
   for (int i = t; i < kH2; i += kThreads) s.b2[i] = w.b2[i];
   for (int i = t; i < kH1; i += kThreads) s.w1b1[i] = w.w1b1[i];
+  for (int i = t; i < kOut * kH2; i += kThreads) (&s.w3[0][0])[i] = w.w3[i];
   if (t < 16) s.b3[t] = t < kOut ? w.b3[t] : 0.f;
 }
 
-__device__ __forceinline__ void load_w2_chunk(Smem& s, const MlpF32& w, int chunk, int buf) {
-  // 128 rows x 64 floats = 2048 x 16 B, 8 per thread
-  const int t = threadIdx.x;
+// Slice q of a tile (chunk q / kSlices, k from kSlice (q % kSlices)) into buffer q % 2.
+__device__ __forceinline__ void load_w2_slice(Smem& s, const MlpF32& w, int q) {
+  const float* src = w.w2t + (size_t)(q % kSlices) * kSlice * kH2 + (q / kSlices) * kChunk;
+  float* dst = &s.w2[q & 1][0][0];
 #pragma unroll
-  for (int q = 0; q < 8; q++) {
-    int idx = t + q * kThreads;  // 0..2047
-    int k = idx >> 4, c4 = idx & 15;
-    cp_async16(&s.w2[buf][k][c4 * 4], w.w2t + (size_t)k * kH2 + chunk * kChunk + c4 * 4);
-  }
+  for (int i = threadIdx.x; i < kSlice * kChunk / 4; i += kThreads)
+    cp_async16(dst + 4 * i, src + (size_t)(i / (kChunk / 4)) * kH2 + 4 * (i % (kChunk / 4)));
   cp_async_commit();
 }
 
-// Evaluates M(r) for s.r[0..127] (caller has written them and synchronized).
+// Evaluates M(r) for s.r[0..63] (caller has written them and synchronized).
 // On return s.y[e][0..8] holds M row-major and the block is synchronized.
 __device__ __forceinline__ void mlp_tile(Smem& s, const MlpF32& w) {
-  const int t = threadIdx.x;
-  load_w2_chunk(s, w, 0, 0);
-  // layer 1: h1[k][e] = tanh(W1[k] . r_e + b1[k])
-  for (int idx = t; idx < kH1 * kTile; idx += kThreads) {
-    const int k = idx / kTile, e = idx % kTile;
-    const float4 wk = s.w1b1[k];
-    const float4 r = s.r[e];
-    s.h1[k][e] = tanh_f32(__fmaf_rn(wk.z, r.z, __fmaf_rn(wk.y, r.y, __fmaf_rn(wk.x, r.x, wk.w))));
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, e0 = kRows * wid;
+  load_w2_slice(s, w, 0);
+  {  // layer 1 of the warp's evaluations: four of them and every eighth unit per thread
+    const int e = e0 + 4 * (lane & 3);
+    const float4 r0 = s.r[e], r1 = s.r[e + 1], r2 = s.r[e + 2], r3 = s.r[e + 3];
+    const f2 x0 = f2_make(r0.x, r1.x), y0 = f2_make(r0.y, r1.y), z0 = f2_make(r0.z, r1.z);
+    const f2 x1 = f2_make(r2.x, r3.x), y1 = f2_make(r2.y, r3.y), z1 = f2_make(r2.z, r3.z);
+#pragma unroll 2
+    for (int k = lane >> 2; k < kH1; k += 8) {
+      const float4 c = s.w1b1[k];
+      const f2 cx = f2_dup(c.x), cy = f2_dup(c.y), cz = f2_dup(c.z), cb = f2_dup(c.w);
+      const f2 a = tanh_f32x2(f2_fma(cz, z0, f2_fma(cy, y0, f2_fma(cx, x0, cb))));
+      const f2 b = tanh_f32x2(f2_fma(cz, z1, f2_fma(cy, y1, f2_fma(cx, x1, cb))));
+      *reinterpret_cast<ulonglong2*>(&s.h1[k][e]) = make_ulonglong2(a.v, b.v);
+    }
+    __syncwarp();
   }
-  const int tn = t & 15, te = t >> 4;   // layer-2 micro tile: evals te*8..+8, units tn*4..+4
-  const int e3 = t & (kTile - 1), og = t >> 7;  // layer-3 owner: eval e3, outputs og*5..
-  const int o0 = og * 5, on = og ? 4 : 5;
-  float y3[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int c = 0; c < kNumChunks; c++) {
-    const int buf = c & 1;
-    cp_async_wait_all();
-    __syncthreads();  // chunk c visible; previous chunk's h2 consumers done
-    if (c + 1 < kNumChunks) load_w2_chunk(s, w, c + 1, buf ^ 1);
-    float acc[8][4];
+  // layer 3: lanes 0-23 take two evaluations (e3, e3 + 1 of the warp's) and three outputs (o3 ..) each
+  const int e3 = 2 * (lane & 7), o3 = lane < 24 ? 3 * (lane >> 3) : 0;
+  f2 y3[3] = {f2_dup(0.f), f2_dup(0.f), f2_dup(0.f)};
+  float(*h2)[kPieceStride] = s.h2[wid];
+#pragma unroll 1
+  for (int c = 0; c < kH2 / kChunk; c++) {
+    f2 acc[kRows / 2][8];  // evaluation pairs x units lane + 32 j of the chunk
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < kRows / 2; i++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+      for (int j = 0; j < 8; j++) acc[i][j] = f2_dup(0.f);
+#pragma unroll 1
+    for (int q = 0; q < kSlices; q++) {
+      cp_async_wait_all();
+      __syncthreads();  // slice visible; every warp is done with the other buffer
+      const int sl = c * kSlices + q;
+      if (sl + 1 < kSlices * (kH2 / kChunk)) load_w2_slice(s, w, sl + 1);
+      const float* wk = &s.w2[sl & 1][0][lane];
+      const ulonglong2* hk = reinterpret_cast<const ulonglong2*>(&s.h1[q * kSlice][e0]);
 #pragma unroll 4
-    for (int k = 0; k < kH1; k++) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&s.h1[k][te * 8]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&s.h1[k][te * 8 + 4]);
-      const float4 b = *reinterpret_cast<const float4*>(&s.w2[buf][k][tn * 4]);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float bv[4] = {b.x, b.y, b.z, b.w};
+      for (int k = 0; k < kSlice; k++) {
+        f2 a[kRows / 2];
 #pragma unroll
-      for (int i = 0; i < 8; i++)
+        for (int i = 0; i < kRows / 4; i++) {
+          const ulonglong2 v = hk[(size_t)k * (kTile / 4) + i];
+          a[2 * i].v = v.x;
+          a[2 * i + 1].v = v.y;
+        }
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = __fmaf_rn(av[i], bv[j], acc[i][j]);
+        for (int j = 0; j < 8; j++) {
+          const f2 b = f2_dup(wk[k * kChunk + 32 * j]);
+#pragma unroll
+          for (int i = 0; i < kRows / 2; i++) acc[i][j] = f2_fma(a[i], b, acc[i][j]);
+        }
+      }
     }
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int n = tn * 4 + j;
-      const float bias = s.b2[c * kChunk + n];
-      float4 v0, v1;
-      v0.x = tanh_f32(__fadd_rn(acc[0][j], bias));
-      v0.y = tanh_f32(__fadd_rn(acc[1][j], bias));
-      v0.z = tanh_f32(__fadd_rn(acc[2][j], bias));
-      v0.w = tanh_f32(__fadd_rn(acc[3][j], bias));
-      v1.x = tanh_f32(__fadd_rn(acc[4][j], bias));
-      v1.y = tanh_f32(__fadd_rn(acc[5][j], bias));
-      v1.z = tanh_f32(__fadd_rn(acc[6][j], bias));
-      v1.w = tanh_f32(__fadd_rn(acc[7][j], bias));
-      *reinterpret_cast<float4*>(&s.h2[n][te * 8]) = v0;
-      *reinterpret_cast<float4*>(&s.h2[n][te * 8 + 4]) = v1;
-    }
-    __syncthreads();
-    // layer 3 partial: y[e3][o] += sum_n h2[n][e3] * W3[o][c*64 + n]
-#pragma unroll 8
-    for (int n = 0; n < kChunk; n++) {
-      const float h = s.h2[n][e3];
+    for (int p = 0; p < kChunk / kPiece; p++) {  // units 64 p .. of the chunk: j = 2 p, 2 p + 1
+      const int n0 = c * kChunk + p * kPiece;
+      __syncwarp();  // the piece before has been read
 #pragma unroll
-      for (int o = 0; o < 5; o++)
-        if (o < on) y3[o] = __fmaf_rn(h, s.w3[o0 + o][c * kChunk + n], y3[o]);
+      for (int j = 0; j < 2; j++) {
+        const f2 bias = f2_dup(s.b2[n0 + 32 * j + lane]);
+#pragma unroll
+        for (int i = 0; i < kRows / 4; i++)
+          *reinterpret_cast<ulonglong2*>(&h2[32 * j + lane][4 * i]) =
+              make_ulonglong2(f2_add(acc[2 * i][2 * p + j], bias).v, f2_add(acc[2 * i + 1][2 * p + j], bias).v);
+      }
+      __syncwarp();
+#pragma unroll 2
+      for (int i = lane; i < kPiece * kRows / 4; i += 32) {  // tanh in place, four evaluations of a unit at a time
+        ulonglong2* v = reinterpret_cast<ulonglong2*>(&h2[i >> 2][4 * (i & 3)]);
+        const ulonglong2 x = *v;
+        *v = make_ulonglong2(tanh_f32x2(f2{x.x}).v, tanh_f32x2(f2{x.y}).v);
+      }
+      __syncwarp();
+#pragma unroll 4
+      for (int n = 0; n < kPiece; n += 4) {
+        const float4 w0 = *reinterpret_cast<const float4*>(&s.w3[o3][n0 + n]);
+        const float4 w1 = *reinterpret_cast<const float4*>(&s.w3[o3 + 1][n0 + n]);
+        const float4 w2 = *reinterpret_cast<const float4*>(&s.w3[o3 + 2][n0 + n]);
+        const float wv[3][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}, {w2.x, w2.y, w2.z, w2.w}};
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          const f2 h = f2{*reinterpret_cast<const uint64_t*>(&h2[n + m][e3])};
+#pragma unroll
+          for (int o = 0; o < 3; o++) y3[o] = f2_fma(h, f2_dup(wv[o][m]), y3[o]);
+        }
+      }
     }
   }
-  // wrapper of python/convert.py:11-20: (y + b3 + I) / |r|, identity for |r| < 1e-5
-  const float4 r = s.r[e3];
-  const float nr = __fsqrt_rn(__fmaf_rn(r.z, r.z, __fmaf_rn(r.y, r.y, __fmul_rn(r.x, r.x))));
-  for (int o = 0; o < on; o++) {
-    const int oo = o0 + o;
-    float v = __fadd_rn(y3[o], s.b3[oo]);
-    if (oo == 0 || oo == 4 || oo == 8) v = __fadd_rn(v, 1.0f);
-    v = __fdiv_rn(v, nr);
-    if (nr < 1e-5f) v = (oo == 0 || oo == 4 || oo == 8) ? 1.0f : 0.0f;
-    s.y[e3][oo] = v;
+  if (lane < 24) {  // wrapper of python/convert.py:11-20: (y + b3 + I) / |r|, identity for |r| < 1e-5
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int e = e0 + e3 + q;
+      const float4 r = s.r[e];
+      const float nr = __fsqrt_rn(__fmaf_rn(r.z, r.z, __fmaf_rn(r.y, r.y, __fmul_rn(r.x, r.x))));
+#pragma unroll
+      for (int o = 0; o < 3; o++) {
+        const bool dg = (o3 + o) % 4 == 0;
+        float v = __fadd_rn(q ? f2_hi(y3[o]) : f2_lo(y3[o]), s.b3[o3 + o]);
+        if (dg) v = __fadd_rn(v, 1.0f);
+        v = __fdiv_rn(v, nr);
+        if (nr < 1e-5f) v = dg ? 1.0f : 0.0f;
+        s.y[e][o3 + o] = v;
+      }
+    }
   }
   __syncthreads();
 }

@@ -95,9 +95,10 @@ struct NaSmem {
   int item;
 };
 
-// One work item = 128 target rows against one source leaf; the symmetrised 3x3
+// One work item = one tile of target rows (simt::kTile) against one source leaf; the symmetrised 3x3
 // 0.5 (M + M^T) of src/DenseDot.cpp:227-243 contracted with the leaf's forces.
-__global__ void __launch_bounds__(simt::kThreads, 1) k_na_dense_rows(NaArgs a, MlpF32 w) {
+__global__ void __launch_bounds__(simt::kThreads, simt::kCtasPerSm)
+    k_na_dense_rows(NaArgs a, MlpF32 w) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   NaSmem& s = *reinterpret_cast<NaSmem*>(smem_raw);
   const int t = threadIdx.x;
@@ -236,7 +237,8 @@ void dense_rows_noalloc(hignn_model* m, double* u_rows, const float* f, const in
   const size_t smem = sizeof(NaSmem);
   HIGNN_CUDA(cudaFuncSetAttribute(k_na_dense_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t nitems = ((nrows + simt::kTile - 1) / simt::kTile) * nleaves;
-  const int grid = (int)(nitems < v.num_sms ? nitems : v.num_sms);
+  const int64_t ctas = (int64_t)simt::kCtasPerSm * v.num_sms;
+  const int grid = (int)(nitems < ctas ? nitems : ctas);
   k_na_dense_rows<<<grid, simt::kThreads, smem, s>>>(a, v.w);
   HIGNN_CHECK_LAUNCH();
   HIGNN_CUDA(cudaMemcpyAsync(u_rows, d_u, sizeof(double) * 3 * nrows, cudaMemcpyDeviceToHost, s));

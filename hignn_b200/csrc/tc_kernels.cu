@@ -46,10 +46,10 @@ constexpr int kParts = tc::kTile / 32;  // rows of a tile per server lane
 // this lane's rows of it as (i, j). Consecutive tiles advance a row by 128 = di nJ + dj.
 struct NearTile {
   PairWork pw;
-  int buf, t0, total, di, dj;
+  int buf, t0, end, di, dj;
   int i[kParts], j[kParts];
-  __device__ __forceinline__ bool last() const { return t0 + tc::kTile >= total; }
-  __device__ __forceinline__ bool valid(int k, int lane) const { return t0 + 32 * k + lane < total; }
+  __device__ __forceinline__ bool last() const { return t0 + tc::kTile >= end; }
+  __device__ __forceinline__ bool valid(int k, int lane) const { return t0 + 32 * k + lane < end; }
 };
 
 // The stream's next close pair (work item `item`) with cleared accumulators b; false at the end of the list.
@@ -61,19 +61,20 @@ __device__ __forceinline__ bool near_fetch(tc::Server& sv, NearStage& G, const N
   const PairWork pw = a.work[item];
   if (lane == 0) item = gridDim.x + atomicAdd(counter, 1);
   __syncwarp();  // every lane is done with the pair that last used accumulators b
-  for (int q = lane; q < 3 * pw.nI; q += 32) (&G.uI[0][0])[q] = 0.f;
-  for (int q = lane; q < 3 * pw.nJ; q += 32) (&G.uJ[0][0])[q] = 0.f;
-  item = __shfl_sync(0xffffffffu, item, 0);
   c.pw = pw;
   c.buf = b;
-  c.t0 = 0;
-  c.total = pw.nI * pw.nJ;
+  c.t0 = pw.first;
+  c.end = pair_end(pw);
+  for (int q = 3 * (pw.first / pw.nJ) + lane; q < 3 * ((c.end - 1) / pw.nJ + 1); q += 32) (&G.uI[0][0])[q] = 0.f;
+  for (int q = lane; q < 3 * pw.nJ; q += 32) (&G.uJ[0][0])[q] = 0.f;
+  item = __shfl_sync(0xffffffffu, item, 0);
   c.di = tc::kTile / pw.nJ;
   c.dj = tc::kTile - c.di * pw.nJ;
 #pragma unroll
   for (int k = 0; k < kParts; k++) {
-    c.i[k] = (32 * k + lane) / pw.nJ;
-    c.j[k] = 32 * k + lane - c.i[k] * pw.nJ;
+    const int flat = pw.first + 32 * k + lane;
+    c.i[k] = flat / pw.nJ;
+    c.j[k] = flat - c.i[k] * pw.nJ;
   }
   __syncwarp();
   return true;
@@ -140,7 +141,7 @@ __device__ __forceinline__ void near_take(tc::Server& sv, NearStage& G, const Ne
   }
   // u_I: the tile's rows cover the targets i0 .. i1; each one's rows are summed over lanes
   const int i0 = c.t0 / c.pw.nJ;
-  const int tail = min(c.t0 + tc::kTile, c.total) - 1, i1 = tail / c.pw.nJ;
+  const int i1 = (min(c.t0 + tc::kTile, c.end) - 1) / c.pw.nJ;
   for (int i = i0; i <= i1; i++) {
     float w[3] = {0.f, 0.f, 0.f};
 #pragma unroll
@@ -160,7 +161,9 @@ __device__ __forceinline__ void near_take(tc::Server& sv, NearStage& G, const Ne
 __device__ __forceinline__ void near_flush(const tc::Server& sv, const NearStage& G, const NearArgs& a,
                                            const PairWork& pw) {
   __syncwarp();
-  for (int q = sv.lane; q < 3 * pw.nI; q += 32) atomicAdd(&a.uI[3 * (size_t)pw.sI + q], (double)(&G.uI[0][0])[q]);
+  const int i0 = pw.first / pw.nJ, i1 = (pair_end(pw) - 1) / pw.nJ;  // targets of the item
+  for (int q = 3 * i0 + sv.lane; q < 3 * (i1 + 1); q += 32)
+    atomicAdd(&a.uI[3 * (size_t)pw.sI + q], (double)(&G.uI[0][0])[q]);
   if (pw.flags & kPairTransposed)
     for (int q = sv.lane; q < 3 * pw.nJ; q += 32) atomicAdd(&a.uJ[3 * (size_t)pw.sJ + q], (double)(&G.uJ[0][0])[q]);
 }
