@@ -35,6 +35,15 @@ constexpr int kPivThreads = 128;
 // slower at N = 1M (287 ms of pivots at 8, 297 at 10, 315 at 12, 337 for the FP64 form)
 constexpr int kPivBlocksF32 = 8;
 constexpr int kApplyThreads = 256;  // the deferred apply: few phases, wider CTAs
+// Where a batch has few blocks, an iteration lasts as long as its largest block: the same kernels then run
+// 512-thread CTAs (the orthogonalisation takes four chunks at once, the cross terms sixteen l). Measured,
+// column + row pivots of one product, 128 against 512 threads: 365 blocks (4,096 spheres, epsilon 1e-5, 100
+// iterations, FP64) 5.8 + 22.9 against 4.3 + 13.8 ms; 750 blocks (5,003 spheres, 1e-2, FP32) 0.48 + 1.01 against
+// 0.49 + 0.89; 1,151 blocks (four products) 2.7 + 5.5 against 3.2 + 4.8; 3,072 blocks (12,289 spheres, FP64)
+// 0.93 + 3.10 against 1.20 + 3.11; 13,453 blocks 3.2 + 5.0 against 4.6 + 6.3. Hence the two lines, in blocks per SM.
+constexpr int kWideThreads = 512;
+constexpr int kWideBlocks = 2;
+constexpr int kWideColLimit = 4, kWideRowLimit = 8;
 
 template <typename T>
 __device__ __forceinline__ T det3(const T* m) {
@@ -303,8 +312,8 @@ __global__ void __launch_bounds__(simt::kThreads, simt::kCtasPerSm)
 }
 
 // Orthogonalise the new column, pick the pivot row, normalise (one CTA per active block).
-template <typename T, int MinBlocks>
-__global__ void __launch_bounds__(kPivThreads, MinBlocks) k_far_col_pivot(FarArgs a) {
+template <typename T, int Threads, int MinBlocks>
+__global__ void __launch_bounds__(Threads, MinBlocks) k_far_col_pivot(FarArgs a) {
   extern __shared__ __align__(16) double dsm[];
   T* qj = reinterpret_cast<T*>(dsm);  // [k][9]
   __shared__ T sv[32], inv[9];
@@ -493,13 +502,13 @@ __device__ void stop_test(const FarArgs& a, int b, const FarBlock& bk, int k, in
 }
 
 // Orthogonalise the new row, pick the next column, stop test, and apply a finished block.
-template <typename T, int MinBlocks>
-__global__ void __launch_bounds__(kPivThreads, MinBlocks) k_far_row_pivot(FarArgs a) {
+template <typename T, int Threads, int MinBlocks>
+__global__ void __launch_bounds__(Threads, MinBlocks) k_far_row_pivot(FarArgs a) {
   extern __shared__ __align__(16) double dsm[];
   T* ci = reinterpret_cast<T*>(dsm);  // [k][9]
   double* mid = dsm + 9 * a.ldr;      // [rank][3]
   double* mid2 = mid + 3 * a.ldr;     // [rank][3]
-  __shared__ T sv[32], cross[8][18], red[32 * 12];
+  __shared__ T sv[32], cross[Threads / 32][18], red[32 * 12];
   __shared__ int si[32];
   __shared__ int s_done, s_rank;
   const int nact = a.ctr[kCtrActive];
@@ -573,8 +582,8 @@ __global__ void __launch_bounds__(kPivThreads, MinBlocks) k_far_row_pivot(FarArg
   const double nu2 = (T)(v[0] * v[6] + v[1] * v[7] + v[2] * v[8] + T(2) * v[9] * v[3] + T(2) * v[10] * v[4] +
                         T(2) * v[11] * v[5]);
   double mu2 = a.state[b].mu2 + nu2;  // every thread tracks the same value; thread 0 stores it
-  // cross terms for l < k - 1 (src/FarDot.cpp:1041-1077), eight l per pass, one warp per l
-  const int nw = blockDim.x >> 5;  // at most 8 (cross)
+  // cross terms for l < k - 1 (src/FarDot.cpp:1041-1077), one warp per l
+  const int nw = blockDim.x >> 5;
   for (int lb = 0; lb < k - 1; lb += nw) {
     const int l = lb + wid;
     if (l < k - 1) {
@@ -648,14 +657,15 @@ __device__ __forceinline__ void warp_sum9(float (&v)[9]) {
     for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
 }
 
-size_t col_smem_f32(int ldr) { return sizeof(float) * (18 * (size_t)ldr + 9 * kPivThreads); }
-size_t row_smem_f32(int ldr) { return sizeof(double) * 6 * (size_t)ldr + col_smem_f32(ldr); }
+size_t col_smem_f32(int ldr, int threads) { return sizeof(float) * (18 * (size_t)ldr + 9 * threads); }
+size_t row_smem_f32(int ldr, int threads) { return sizeof(double) * 6 * (size_t)ldr + col_smem_f32(ldr, threads); }
 
-__global__ void __launch_bounds__(kPivThreads, kPivBlocksF32) k_far_col_pivot_f32(FarArgs a) {
+template <int Threads, int MinBlocks>
+__global__ void __launch_bounds__(Threads, MinBlocks) k_far_col_pivot_f32(FarArgs a) {
   extern __shared__ __align__(16) float fsm[];
   float* qj = fsm;             // [k][9]: Q_l[j_k]
   float* xo = qj + 9 * a.ldr;  // [k - 1][9]: cross terms of the orthogonalised column with C_l
-  float* cs = xo + 9 * a.ldr;  // [128][9]: the chunk's orthogonalised entries
+  float* cs = xo + 9 * a.ldr;  // [Threads][9]: the chunk's orthogonalised entries
   __shared__ float sv[32], inv[9], red[32 * 6];
   __shared__ int si[32];
   const int nact = a.ctr[kCtrActive];
@@ -799,13 +809,14 @@ __global__ void __launch_bounds__(kPivThreads, kPivBlocksF32) k_far_col_pivot_f3
   }
 }
 
-__global__ void __launch_bounds__(kPivThreads, kPivBlocksF32) k_far_row_pivot_f32(FarArgs a) {
+template <int Threads, int MinBlocks>
+__global__ void __launch_bounds__(Threads, MinBlocks) k_far_row_pivot_f32(FarArgs a) {
   extern __shared__ __align__(16) double dsm[];
   double* mid = dsm;                                       // [rank][3] (apply)
   double* mid2 = mid + 3 * a.ldr;                          // [rank][3]
   float* ci = reinterpret_cast<float*>(mid2 + 3 * a.ldr);  // [k][9]: C_l[i_k]
   float* xq = ci + 9 * a.ldr;                              // [k - 1][9]: cross terms of Q_k with Q_l
-  float* qs = xq + 9 * a.ldr;                              // [128][9]: the chunk's orthogonalised entries
+  float* qs = xq + 9 * a.ldr;                              // [Threads][9]: the chunk's orthogonalised entries
   __shared__ float sv[32], red[32 * 6];
   __shared__ int si[32];
   __shared__ int s_done, s_rank;
@@ -1021,6 +1032,7 @@ void far_iteration(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, cons
   const size_t row_smem = sizeof(double) * (9 + 3 + 3) * a.ldr;
   const size_t col_smem = sizeof(double) * 9 * a.ldr;
   const int piv_grid = a.nb < 16 * num_sms ? a.nb : 16 * num_sms;  // grid-stride over active blocks
+  const bool wide_col = a.nb <= kWideColLimit * num_sms, wide_row = a.nb <= kWideRowLimit * num_sms;
   mark();
   k_far_active<<<1, 1024, 0, s>>>(a);
   mark();
@@ -1031,10 +1043,14 @@ void far_iteration(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, cons
   else
     k_far_eval<<<simt::kCtasPerSm * num_sms, simt::kThreads, eval_smem, s>>>(a, w, 0);
   mark();
-  if (a.fast_pivots)
-    k_far_col_pivot_f32<<<piv_grid, kPivThreads, col_smem_f32(a.ldr), s>>>(a);
+  if (a.fast_pivots && wide_col)
+    k_far_col_pivot_f32<kWideThreads, kWideBlocks><<<a.nb, kWideThreads, col_smem_f32(a.ldr, kWideThreads), s>>>(a);
+  else if (a.fast_pivots)
+    k_far_col_pivot_f32<kPivThreads, kPivBlocksF32><<<piv_grid, kPivThreads, col_smem_f32(a.ldr, kPivThreads), s>>>(a);
+  else if (wide_col)
+    k_far_col_pivot<double, kWideThreads, kWideBlocks><<<a.nb, kWideThreads, col_smem, s>>>(a);
   else
-    k_far_col_pivot<double, 8><<<piv_grid, kPivThreads, col_smem, s>>>(a);
+    k_far_col_pivot<double, kPivThreads, 8><<<piv_grid, kPivThreads, col_smem, s>>>(a);
   mark();
   if (student)
     launch_far_student(a, student, 1, err, num_sms, s);
@@ -1043,10 +1059,14 @@ void far_iteration(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, cons
   else
     k_far_eval<<<simt::kCtasPerSm * num_sms, simt::kThreads, eval_smem, s>>>(a, w, 1);
   mark();
-  if (a.fast_pivots)
-    k_far_row_pivot_f32<<<piv_grid, kPivThreads, row_smem_f32(a.ldr), s>>>(a);
+  if (a.fast_pivots && wide_row)
+    k_far_row_pivot_f32<kWideThreads, kWideBlocks><<<a.nb, kWideThreads, row_smem_f32(a.ldr, kWideThreads), s>>>(a);
+  else if (a.fast_pivots)
+    k_far_row_pivot_f32<kPivThreads, kPivBlocksF32><<<piv_grid, kPivThreads, row_smem_f32(a.ldr, kPivThreads), s>>>(a);
+  else if (wide_row)
+    k_far_row_pivot<double, kWideThreads, kWideBlocks><<<a.nb, kWideThreads, row_smem, s>>>(a);
   else
-    k_far_row_pivot<double, 8><<<piv_grid, kPivThreads, row_smem, s>>>(a);
+    k_far_row_pivot<double, kPivThreads, 8><<<piv_grid, kPivThreads, row_smem, s>>>(a);
   mark();
   HIGNN_CHECK_LAUNCH();
 }
@@ -1057,10 +1077,14 @@ void far_batch_start(const FarArgs& a, cudaStream_t s) {
   const size_t row_smem = sizeof(double) * (9 + 3 + 3) * a.ldr;
   const size_t col_smem = sizeof(double) * 9 * a.ldr;
   set_max_dynamic_smem(k_far_eval, eval_smem, s);
-  set_max_dynamic_smem(k_far_row_pivot<double, 8>, row_smem, s);
-  set_max_dynamic_smem(k_far_col_pivot<double, 8>, col_smem, s);
-  set_max_dynamic_smem(k_far_row_pivot_f32, row_smem_f32(a.ldr), s);
-  set_max_dynamic_smem(k_far_col_pivot_f32, col_smem_f32(a.ldr), s);
+  set_max_dynamic_smem(k_far_row_pivot<double, kPivThreads, 8>, row_smem, s);
+  set_max_dynamic_smem(k_far_col_pivot<double, kPivThreads, 8>, col_smem, s);
+  set_max_dynamic_smem(k_far_row_pivot<double, kWideThreads, kWideBlocks>, row_smem, s);
+  set_max_dynamic_smem(k_far_col_pivot<double, kWideThreads, kWideBlocks>, col_smem, s);
+  set_max_dynamic_smem(k_far_row_pivot_f32<kPivThreads, kPivBlocksF32>, row_smem_f32(a.ldr, kPivThreads), s);
+  set_max_dynamic_smem(k_far_col_pivot_f32<kPivThreads, kPivBlocksF32>, col_smem_f32(a.ldr, kPivThreads), s);
+  set_max_dynamic_smem(k_far_row_pivot_f32<kWideThreads, kWideBlocks>, row_smem_f32(a.ldr, kWideThreads), s);
+  set_max_dynamic_smem(k_far_col_pivot_f32<kWideThreads, kWideBlocks>, col_smem_f32(a.ldr, kWideThreads), s);
   k_far_init<<<(a.nb + 255) / 256, 256, 0, s>>>(a);
   HIGNN_CHECK_LAUNCH();
 }
