@@ -20,14 +20,19 @@
 // shared nor tensor memory.
 // Layer 2 is cut into sixteen chunks of 128 outputs (eight per pass); the epilogue releases the
 // layer-2 accumulator as soon as it has read it, then writes the chunk's tanh'd FP16 values to a
-// shared-memory buffer (two, in turn) that is the K-slice of layer 3 (N = 256). The MMA lane
+// shared-memory buffer (two, in turn) that is the K-slice of layer 3 (N = 256). The MMA warp
 // interleaves the chunks, L2(g + 1) before L3(g), so the tensor pipe has a layer-3 slice to run
 // while the epilogue turns an accumulator around.
 // The weights (1.6 MB of FP16) stream through a five-deep ring of 32 KB shared-memory stages,
 // filled by bulk copies from a host-built image laid out in the order the MMAs consume it.
 //
+// The MMA warp runs its loop warp-uniformly and one elected lane issues, and a wait that is already over reads
+// no clock: 9.95 -> 8.70 ms for 4.41 M triplets (0.49 of the measured bf16 peak). One arrival per
+// epilogue warp instead of one per thread was slower (15 ms: the compiler then spills twice as much around the
+// epilogue's constants).
+//
 // CTA = 18 warps: 0-15 epilogue (warp w reaches TMEM lanes 32 (w % 4) + 0..31, so row
-// e = 32 (w % 4) + lane has four threads, part p = w / 4), 16 MMA lane, 17 producer.
+// e = 32 (w % 4) + lane has four threads, part p = w / 4), 16 MMA warp, 17 producer.
 // Every wait is bounded (about two seconds of clock); on a timeout the CTA records an error,
 // stops, lets its copies and MMAs drain and frees its tensor memory.
 #include <cuda_fp16.h>
@@ -76,6 +81,7 @@ static_assert(sizeof(TbConst) + 128 <= 32764, "three-body kernel parameters exce
 
 __device__ __forceinline__ bool wait_bar(uint64_t* b, uint32_t parity, int* abort_flag, int* err, int code,
                                          bool honour_abort = true) {
+  if (tc::mbar_try(b, parity)) return true;  // no clock read where the wait is already over
   const long long t0 = clock64();
   while (!mbar_try_sleep(b, parity, 20000u)) {
     if (honour_abort && *(volatile int*)abort_flag) return false;
@@ -86,6 +92,11 @@ __device__ __forceinline__ bool wait_bar(uint64_t* b, uint32_t parity, int* abor
     }
   }
   return true;
+}
+
+// The same for a whole warp: every lane gets the same answer.
+__device__ __forceinline__ bool warp_wait_bar(uint64_t* b, uint32_t parity, int* abort_flag, int* err, int code) {
+  return __all_sync(0xffffffffu, wait_bar(b, parity, abort_flag, err, code));
 }
 
 __device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
@@ -363,8 +374,11 @@ struct Epi {
   }
 };
 
-// ------------------------------------------------------------------ MMA lane
-struct MmaLaneTb {
+// ------------------------------------------------------------------ MMA warp
+// The whole warp runs the loop, so that addresses and descriptors are warp-uniform (a lane that branches
+// off by itself needs ~130 cycles per MMA to bring its operands into uniform registers), and one
+// elected lane issues.
+struct MmaWarpTb {
   TbSmem& s;
   int* err;
   uint32_t tb;
@@ -375,15 +389,14 @@ struct MmaLaneTb {
   __device__ __forceinline__ bool wait(uint64_t* b, uint32_t parity, int code) {
     if (!ok) return false;
     const long long t0 = clock64();
-    ok = wait_bar(b, parity, &s.abort_flag, err, code);
+    ok = warp_wait_bar(b, parity, &s.abort_flag, err, code);
     waited[code == 50 ? 0 : code == 51 ? 1 : code == 54 ? 3 : 2] += clock64() - t0;
     if (ok) fence_after();
     return ok;
   }
   __device__ __forceinline__ bool stage_ready() { return wait(&s.ring_full[S % kRing], (S / kRing) & 1, 51); }
-  __device__ __forceinline__ void stage_done() {
+  __device__ __forceinline__ void stage_done() {  // by the issuing lane
     mma_commit(&s.ring_empty[S % kRing]);
-    S++;
   }
   // layer-2 chunk g (global chunk index; the accumulator is free once the epilogue has read
   // chunk g - 1): A = layer 1 in tensor memory, two 32 KB stages of W2 (K 0-127, 128-255)
@@ -393,15 +406,19 @@ struct MmaLaneTb {
     for (uint32_t st = 0; st < 2; st++) {
       if (!stage_ready()) return false;
       const uint64_t b0 = sdesc(saddr(s.ring[S % kRing]));
+      if (tc::elect_one()) {
 #pragma unroll
-      for (uint32_t i = 0; i < 8; i++) {
-        const uint32_t k16 = 8 * st + i;  // K = 16 k16 .. + 15
-        const uint64_t bd = b0 + (i >> 2) * (16384 >> 4) + (i & 3) * 2;
-        tc::mma_ts(tb + kOffD2, tb + kOffA1 + 8 * k16, bd, id, k16 != 0);
+        for (uint32_t i = 0; i < 8; i++) {
+          const uint32_t k16 = 8 * st + i;  // K = 16 k16 .. + 15
+          const uint64_t bd = b0 + (i >> 2) * (16384 >> 4) + (i & 3) * 2;
+          tc::mma_ts(tb + kOffD2, tb + kOffA1 + 8 * k16, bd, id, k16 != 0);
+        }
+        stage_done();
+        if (st == 1) mma_commit(&s.d2_full);
       }
-      stage_done();
+      __syncwarp();
+      S++;
     }
-    mma_commit(&s.d2_full);
     return true;
   }
   // layer-3 K-slice of chunk g (local chunk c, pass P) into D3: N = 256, two 32 KB stages of W3
@@ -413,11 +430,15 @@ struct MmaLaneTb {
     for (uint32_t kb = 0; kb < 2; kb++) {
       if (!stage_ready()) return false;
       const uint64_t a0 = sdesc(saddr(s.act2[g & 1][kb])), b0 = sdesc(saddr(s.ring[S % kRing]));
+      if (tc::elect_one()) {
 #pragma unroll
-      for (uint32_t kk = 0; kk < 4; kk++) mma_ss(tb + kOffD3, a0 + 2 * kk, b0 + 2 * kk, id, (c | kb | kk) != 0);
-      stage_done();
+        for (uint32_t kk = 0; kk < 4; kk++) mma_ss(tb + kOffD3, a0 + 2 * kk, b0 + 2 * kk, id, (c | kb | kk) != 0);
+        stage_done();
+        if (kb == 1 && c == 7) mma_commit(&s.d3_full);
+      }
+      __syncwarp();
+      S++;
     }
-    if (c == 7) mma_commit(&s.d3_full);
     return true;
   }
 
@@ -428,11 +449,15 @@ struct MmaLaneTb {
     if (!stage_ready()) return false;
     const uint64_t b0 = sdesc(saddr(s.ring[S % kRing]));
     const uint32_t id = idesc_f16(128, 16);
+    if (tc::elect_one()) {
 #pragma unroll
-    for (uint32_t k16 = 0; k16 < 16; k16++)
-      tc::mma_ts(tb + kOffD4, tb + kOffA3 + 8 * k16, b0 + (k16 >> 2) * (2048 >> 4) + (k16 & 3) * 2, id, k16 != 0);
-    stage_done();
-    mma_commit(&s.d4_full);
+      for (uint32_t k16 = 0; k16 < 16; k16++)
+        tc::mma_ts(tb + kOffD4, tb + kOffA3 + 8 * k16, b0 + (k16 >> 2) * (2048 >> 4) + (k16 & 3) * 2, id, k16 != 0);
+      stage_done();
+      mma_commit(&s.d4_full);
+    }
+    __syncwarp();
+    S++;
     return true;
   }
 
@@ -453,9 +478,12 @@ struct MmaLaneTb {
       if (ok) l4(2 * k + 1);
     }
     // let every issued MMA finish before the tensor memory is freed
-    mma_commit(&s.drain);
-    wait_bar(&s.drain, 0, &s.abort_flag, err, 55, false);
-    if (prof) {
+    if (tc::elect_one()) {
+      mma_commit(&s.drain);
+      wait_bar(&s.drain, 0, &s.abort_flag, err, 55, false);
+    }
+    __syncwarp();
+    if (prof && (threadIdx.x & 31) == 0) {
       for (int i = 0; i < 4; i++) atomicAdd(&prof[i], (unsigned long long)waited[i]);
       atomicAdd(&prof[4], (unsigned long long)(clock64() - start));
     }
@@ -534,10 +562,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     ep.tlane = s.tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
     ep.run(ntiles);
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
-      MmaLaneTb ml{s, err, s.tmem_base};
-      ml.run(ntiles, prof);
-    }
+    MmaWarpTb mw{s, err, __shfl_sync(0xffffffffu, s.tmem_base, 0)};
+    mw.run(ntiles, prof);
   } else if (warp == kProdWarp && lane == 0) {
     producer(s, w.img, ntiles, err, prof);
   }
