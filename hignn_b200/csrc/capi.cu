@@ -201,7 +201,21 @@ void require_device(hignn_model* m) {
   HIGNN_CUDA(cudaSetDevice(m->device));
 }
 
-constexpr int64_t kItemEvals = 128;  // near-field work items are cut at multiples of a tile
+constexpr int64_t kItemEvals = 128;  // work items are cut at multiples of a tile
+
+// Evaluations per work item for `evals` evaluations in about `items` items.
+int64_t item_evals(double evals, int items) {
+  return ((int64_t)(evals / std::max(1, items)) / kItemEvals + 1) * kItemEvals;
+}
+// The pair w as work items of at most per_item evaluations.
+void cut_pair(hignn::PairWork w, int64_t per_item, std::vector<hignn::PairWork>& work) {
+  const int64_t total = (int64_t)w.nI * w.nJ;
+  for (int64_t e = 0; e < total; e += per_item) {
+    w.first = (int32_t)e;
+    w.count = (int32_t)std::min(per_item, total - e);
+    work.push_back(w);
+  }
+}
 
 // Builds the tree and lists of m->xyz and, on a device model, uploads the tree-order positions
 // and the close work list. Everything is built and checked before the model changes: a tree that
@@ -317,7 +331,7 @@ void build_structures(hignn_model* m) {
     const auto& J = m->tree.nodes[m->lists.closeJ[q]];
     evals += (I.end - I.start) * (J.end - J.start);
   }
-  const int64_t per_item = (evals / (8 * 2 * (int64_t)std::max(1, m->num_sms)) / kItemEvals + 1) * kItemEvals;
+  const int64_t per_item = item_evals((double)evals, 8 * 2 * m->num_sms);
   m->close_item0.resize(nclose + 1);
   for (size_t q = 0; q < nclose; q++) {
     const auto& I = m->tree.nodes[m->lists.closeI[q]];
@@ -329,12 +343,7 @@ void build_structures(hignn_model* m) {
     w.nJ = (int32_t)(J.end - J.start);
     w.flags = (m->use_symmetry && m->lists.closeJ[q] > m->lists.closeI[q]) ? hignn::kPairTransposed : 0;
     m->close_item0[q] = (int64_t)work.size();
-    const int64_t total = (int64_t)w.nI * w.nJ;
-    for (int64_t e = 0; e < total; e += per_item) {
-      w.first = (int32_t)e;
-      w.count = (int32_t)std::min(per_item, total - e);
-      work.push_back(w);
-    }
+    cut_pair(w, per_item, work);
   }
   m->close_item0[nclose] = (int64_t)work.size();
   m->stats.close_evals = evals;
@@ -1834,6 +1843,8 @@ int hignn_dense_rows(hignn_model* m, double* u_rows, const float* f, const int64
       pos[q] = (int32_t)m->inv_perm[rows[q]];
     }
     std::vector<hignn::PairWork> work;
+    // few rows: items cut into runs of evaluations (about eight per SM), as the close pairs are
+    const int64_t per_item = item_evals((double)nrows * (double)m->n, 8 * m->num_sms);
     for (int64_t c0 = 0; c0 < nrows; c0 += 128)
       for (int64_t J : lv) {
         const auto& b = m->tree.nodes[J];
@@ -1843,7 +1854,7 @@ int hignn_dense_rows(hignn_model* m, double* u_rows, const float* f, const int64
         w.sJ = (int32_t)b.start;
         w.nJ = (int32_t)(b.end - b.start);
         w.flags = hignn::kPairSymmetrize;
-        work.push_back(w);
+        cut_pair(w, per_item, work);
       }
     m->tmp_pos.ensure(sizeof(int32_t) * nrows);
     m->tmp_x.ensure(sizeof(float4) * nrows);

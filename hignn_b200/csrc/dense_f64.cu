@@ -7,13 +7,20 @@
 // list as the FP32 dense rows (PairWork items flagged kPairSymmetrize: up to 128 gathered target
 // rows against one source leaf of up to kMaxLeaf particles).
 //
-// One persistent CTA per SM, 256 threads, tiles of 128 evaluations:
+// One persistent CTA of sixteen warps per SM, tiles of 128 evaluations. Layers 2 and 3 are FP64
+// mma.sync (m8n8k4), which reach the FP64 pipe's 64 FMA per clock per SM with 12 clocks of shared-memory
+// reads per 128 of the pipe; register-tiled scalar FMAs need three times the reads.
 //   layer 1: h1[k][e] = tanh(W1[k] . r_e + b1[k]) (128 x 128 doubles in shared memory);
-//   layer 2: eight chunks of 64 hidden units, each a 128 x 64 x 128 register-tiled DGEMM (8
-//            evaluations x 4 units per thread) on one W2^T chunk staged in shared memory as
-//            doubles; the chunk buffer then receives tanh(acc + b2) as [unit][evaluation];
-//   layer 3: y[e][o] += sum_n h2[n][e] W3[o][n], W3 read through the read-only cache;
+//   layer 2: eight chunks of 64 hidden units, 32 evaluations x 16 units per warp, on one W2^T chunk
+//            staged in shared memory as doubles (the next chunk's values are fetched meanwhile);
+//            the chunk buffer then receives tanh(acc + b2) as [unit][evaluation];
+//   layer 3: warp w accumulates the outputs of evaluations 8 w .. 8 w + 7 (columns 0-8 of 16),
+//            W3 read through the read-only cache;
 //   wrapper: (y + b3 + I) / |r|, identity below |r| = 1e-5 (python/convert.py:11-20).
+// Both shared arrays have row strides of 4 mod 16 doubles: a fragment's 4 k x 8 rows then hit every bank once
+// per half warp. The bound is the FP64 pipe: 70,528 FMA and 640 tanh per evaluation (1,100 clocks of FMA, about 440
+// of tanh with sixteen warps). Measured (one B200, 100 rows x 65,536 sources): 54.0 ms, against 94.4 ms of 8 x 4
+// scalar FMAs per thread in eight warps and whole (rows, leaf) items.
 #include "common.h"
 #include "kernels.h"
 
@@ -21,88 +28,118 @@ namespace hignn {
 
 namespace {
 
-constexpr int kF64Threads = 256;
+constexpr int kF64Warps = 16;
+constexpr int kF64Threads = 32 * kF64Warps;
 constexpr int kF64Tile = 128;
 constexpr int kF64Chunk = 64;
-constexpr int kH2Stride = kF64Tile + 2;  // h2 rows padded: the [unit][evaluation] stores spread over the banks
+constexpr int kH1Stride = kF64Tile + 4, kH2Stride = kF64Tile + 4, kW2Stride = kF64Chunk + 4;
+constexpr int kF64Out = 10;
+static_assert(kF64Tile == 8 * kF64Warps, "layer 3 gives a warp eight evaluations");
 
 struct F64Smem {
-  double h1[kH1][kF64Tile];          // 128 KB
-  double buf[kF64Chunk * kH2Stride];  // 65 KB: W2^T chunk [k][n], then h2 [n][e] (row stride kH2Stride)
+  double h1[kH1 * kH1Stride];   // 132 KB, [k][e]
+  double buf[kH1 * kW2Stride];  // 68 KB: W2^T chunk [k][n], then h2 [n][e]
   double r[kF64Tile][3];
-  double y[kF64Tile][kOut];
+  double y[kF64Tile][kF64Out];
   double uI[kF64Tile][3];
-  float4 xI[kF64Tile];
-  float4 xJ[kMaxLeaf], fJ[kMaxLeaf];
-  int16_t ei[kF64Tile], ej[kF64Tile];
   int item;
 };
 static_assert(sizeof(F64Smem) <= 232448, "FP64 dense-rows shared memory exceeds 227 KB per CTA");
+static_assert(kF64Chunk * kH2Stride <= kH1 * kW2Stride, "h2 does not fit the chunk buffer");
+
+// D += A B: lane l holds A[l / 4][l % 4], B[l % 4][l / 4] and D[l / 4][2 (l % 4) + {0, 1}].
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
 
 __device__ __forceinline__ void f64_tile(F64Smem& s, const MlpF32& w) {
-  const int t = threadIdx.x;
-  // layer 1
-  for (int idx = t; idx < kH1 * kF64Tile; idx += kF64Threads) {
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const int fr = lane >> 2, fk = lane & 3;  // a fragment's row (or column) and k of this lane
+  constexpr int kFetch = kH1 * kF64Chunk / kF64Threads;
+  float pre[kFetch];  // the next W2^T chunk
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int q = 0; q < kFetch; q++) {
+      const int idx = t + q * kF64Threads;
+      pre[q] = __ldg(&w.w2t[(size_t)(idx / kF64Chunk) * kH2 + c * kF64Chunk + idx % kF64Chunk]);
+    }
+  };
+  fetch(0);
+  for (int idx = t; idx < kH1 * kF64Tile; idx += kF64Threads) {  // layer 1
     const int k = idx / kF64Tile, e = idx % kF64Tile;
     const float4 wk = __ldg(&w.w1b1[k]);
     const double z = (double)wk.w + (double)wk.x * s.r[e][0] + (double)wk.y * s.r[e][1] + (double)wk.z * s.r[e][2];
-    s.h1[k][e] = tanh(z);
+    s.h1[k * kH1Stride + e] = tanh(z);
   }
-  const int tn = t & 15, te = t >> 4;            // layer-2 micro tile: evals te*8..+8, units tn*4..+4
-  const int e3 = t & (kF64Tile - 1), og = t >> 7;  // layer-3 owner: eval e3, outputs og*5..
-  const int o0 = og * 5, on = og ? 4 : 5;
-  double y3[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  const int em = 32 * (wid & 3), un = 16 * (wid >> 2);  // layer 2: the warp's evaluations and units of a chunk
+  double y3[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll 1
   for (int c = 0; c < kH2 / kF64Chunk; c++) {
     __syncthreads();  // layer 1 done / previous chunk's h2 readers done
-    for (int idx = t; idx < kH1 * kF64Chunk; idx += kF64Threads) {
-      const int k = idx / kF64Chunk, n = idx % kF64Chunk;
-      s.buf[idx] = (double)__ldg(&w.w2t[(size_t)k * kH2 + c * kF64Chunk + n]);
+#pragma unroll
+    for (int q = 0; q < kFetch; q++) {
+      const int idx = t + q * kF64Threads;
+      s.buf[idx / kF64Chunk * kW2Stride + idx % kF64Chunk] = (double)pre[q];
     }
     __syncthreads();
-    double acc[8][4];
+    if (c + 1 < kH2 / kF64Chunk) fetch(c + 1);
+    double acc[4][2][2];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < 4; i++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
-#pragma unroll 2
-    for (int k = 0; k < kH1; k++) {
-      const double2* ap = reinterpret_cast<const double2*>(&s.h1[k][te * 8]);
-      const double2* bp = reinterpret_cast<const double2*>(&s.buf[k * kF64Chunk + tn * 4]);
-      const double2 a0 = ap[0], a1 = ap[1], a2 = ap[2], a3 = ap[3];
-      const double2 b0 = bp[0], b1 = bp[1];
-      const double av[8] = {a0.x, a0.y, a1.x, a1.y, a2.x, a2.y, a3.x, a3.y};
-      const double bv[4] = {b0.x, b0.y, b1.x, b1.y};
+      for (int j = 0; j < 2; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+    const double* ap = s.h1 + fk * kH1Stride + em + fr;
+    const double* bp = s.buf + fk * kW2Stride + un + fr;
+#pragma unroll 4
+    for (int k = 0; k < kH1; k += 4) {
+      double a[4], b[2];
 #pragma unroll
-      for (int i = 0; i < 8; i++)
+      for (int i = 0; i < 4; i++) a[i] = ap[k * kH1Stride + 8 * i];
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+      for (int j = 0; j < 2; j++) b[j] = bp[k * kW2Stride + 8 * j];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) dmma(acc[i][j], a[i], b[j]);
     }
-    __syncthreads();  // every thread is done with the W2 chunk: the buffer takes h2
+    __syncthreads();  // every warp is done with the W2 chunk: the buffer takes h2
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int n = tn * 4 + j;
-      const double bias = (double)__ldg(&w.b2[c * kF64Chunk + n]);
+    for (int j = 0; j < 2; j++)
 #pragma unroll
-      for (int i = 0; i < 8; i++) s.buf[n * kH2Stride + te * 8 + i] = tanh(acc[i][j] + bias);
-    }
+      for (int h = 0; h < 2; h++) {
+        const int n = un + 8 * j + 2 * fk + h;
+        const double bias = (double)__ldg(&w.b2[c * kF64Chunk + n]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) s.buf[n * kH2Stride + em + 8 * i + fr] = tanh(acc[i][j][h] + bias);
+      }
     __syncthreads();
-    for (int n = 0; n < kF64Chunk; n++) {
-      const double h = s.buf[n * kH2Stride + e3];
-#pragma unroll
-      for (int o = 0; o < 5; o++)
-        if (o < on) y3[o] = fma(h, (double)__ldg(&w.w3[(o0 + o) * kH2 + c * kF64Chunk + n]), y3[o]);
+    const double* hp = s.buf + fk * kH2Stride + 8 * wid + fr;
+#pragma unroll 4
+    for (int n = 0; n < kF64Chunk; n += 4) {
+      const double a = hp[n * kH2Stride];
+      const int col = c * kF64Chunk + n + fk;
+      dmma(y3[0], a, (double)__ldg(&w.w3[fr * kH2 + col]));
+      dmma(y3[1], a, fr == 0 ? (double)__ldg(&w.w3[8 * kH2 + col]) : 0.0);
     }
   }
-  const double rx = s.r[e3][0], ry = s.r[e3][1], rz = s.r[e3][2];
-  const double nr = sqrt(rx * rx + ry * ry + rz * rz);
-  for (int o = 0; o < on; o++) {
-    const int oo = o0 + o;
-    double v = y3[o] + (double)__ldg(&w.b3[oo]);
-    const bool dg = (oo == 0 || oo == 4 || oo == 8);
-    if (dg) v += 1.0;
-    v = v / nr;
-    if (nr < 1e-5) v = dg ? 1.0 : 0.0;
-    s.y[e3][oo] = v;
+  s.y[8 * wid + fr][2 * fk] = y3[0][0];
+  s.y[8 * wid + fr][2 * fk + 1] = y3[0][1];
+  if (fk == 0) s.y[8 * wid + fr][8] = y3[1][0];
+  __syncthreads();
+  for (int e = t; e < kF64Tile; e += kF64Threads) {
+    const double rx = s.r[e][0], ry = s.r[e][1], rz = s.r[e][2];
+    const double nr = sqrt(rx * rx + ry * ry + rz * rz);
+#pragma unroll
+    for (int o = 0; o < kOut; o++) {
+      double v = s.y[e][o] + (double)__ldg(&w.b3[o]);
+      const bool dg = o % 4 == 0;
+      if (dg) v += 1.0;
+      v = v / nr;
+      if (nr < 1e-5) v = dg ? 1.0 : 0.0;
+      s.y[e][o] = v;
+    }
   }
   __syncthreads();
 }
@@ -118,37 +155,22 @@ __global__ void __launch_bounds__(kF64Threads, 1) k_dense_rows_f64(NearArgs a, M
     const int item = s.item;
     if (item >= a.nwork) break;
     const PairWork pw = a.work[item];
-    for (int i = t; i < pw.nI; i += kF64Threads) {
-      s.xI[i] = a.xI[pw.sI + i];
-      s.uI[i][0] = s.uI[i][1] = s.uI[i][2] = 0.0;
-    }
-    for (int j = t; j < pw.nJ; j += kF64Threads) {
-      s.xJ[j] = a.xJ[pw.sJ + j];
-      s.fJ[j] = a.fJ[pw.sJ + j];
-    }
-    __syncthreads();
-    const int total = pw.nI * pw.nJ;
-    for (int t0 = 0; t0 < total; t0 += kF64Tile) {
+    const int end = pair_end(pw);
+    const int i0 = pw.first / pw.nJ, i1 = (end - 1) / pw.nJ;  // targets of the item
+    for (int i = i0 + t; i <= i1; i += kF64Threads) s.uI[i][0] = s.uI[i][1] = s.uI[i][2] = 0.0;
+    for (int t0 = pw.first; t0 < end; t0 += kF64Tile) {
+      const int flat = t0 + t;
+      const bool valid = t < kF64Tile && flat < end;
+      const int i = valid ? flat / pw.nJ : 0, j = valid ? flat - i * pw.nJ : 0;
       if (t < kF64Tile) {
-        const int flat = t0 + t;
-        if (flat < total) {
-          const int i = flat / pw.nJ, j = flat - (flat / pw.nJ) * pw.nJ;
-          const float4 xi = s.xI[i], xj = s.xJ[j];
-          s.r[t][0] = (double)xj.x - (double)xi.x;
-          s.r[t][1] = (double)xj.y - (double)xi.y;
-          s.r[t][2] = (double)xj.z - (double)xi.z;
-          s.ei[t] = (int16_t)i;
-          s.ej[t] = (int16_t)j;
-        } else {
-          s.r[t][0] = 1.0;
-          s.r[t][1] = s.r[t][2] = 0.0;
-          s.ei[t] = -1;
-        }
+        const float4 xi = __ldg(&a.xI[pw.sI + i]), xj = __ldg(&a.xJ[pw.sJ + j]);
+        s.r[t][0] = valid ? (double)xj.x - (double)xi.x : 1.0;
+        s.r[t][1] = valid ? (double)xj.y - (double)xi.y : 0.0;
+        s.r[t][2] = valid ? (double)xj.z - (double)xi.z : 0.0;
       }
       __syncthreads();
       f64_tile(s, w);
-      if (t < kF64Tile && s.ei[t] >= 0) {
-        const int i = s.ei[t], j = s.ej[t];
+      if (valid) {
         double M[9];
 #pragma unroll
         for (int q = 0; q < 9; q++) M[q] = s.y[t][q];
@@ -160,7 +182,7 @@ __global__ void __launch_bounds__(kF64Threads, 1) k_dense_rows_f64(NearArgs a, M
             M[3 * r + c] = v;
             M[3 * c + r] = v;
           }
-        const float4 fj = s.fJ[j];
+        const float4 fj = __ldg(&a.fJ[pw.sJ + j]);
         const double fx = fj.x, fy = fj.y, fz = fj.z;
         atomicAdd(&s.uI[i][0], M[0] * fx + M[1] * fy + M[2] * fz);
         atomicAdd(&s.uI[i][1], M[3] * fx + M[4] * fy + M[5] * fz);
@@ -168,7 +190,8 @@ __global__ void __launch_bounds__(kF64Threads, 1) k_dense_rows_f64(NearArgs a, M
       }
     }
     __syncthreads();
-    for (int q = t; q < 3 * pw.nI; q += kF64Threads) atomicAdd(&a.uI[3 * (size_t)pw.sI + q], (&s.uI[0][0])[q]);
+    for (int q = 3 * i0 + t; q < 3 * (i1 + 1); q += kF64Threads)
+      atomicAdd(&a.uI[3 * (size_t)pw.sI + q], (&s.uI[0][0])[q]);
   }
 }
 
