@@ -162,6 +162,7 @@ struct hignn_model {
   std::vector<int32_t> rank_hint;
   bool hint_valid = false;
   int hint_precision = -1, hint_max_iter = -1;
+  int hint_max = 1;  // largest rank of this shard's blocks when ranks were last recorded; kept across rebuilds
   double hint_epsilon = -1.0;
 
   hignn_stats stats{};
@@ -284,7 +285,7 @@ void build_structures(hignn_model* m) {
   m->lists = std::move(lists);
   m->lists_sym = m->use_symmetry;
   m->lists_max_rel = m->max_relative_coord;
-  if (carry) {  // hints for the new lists; -1 = not known (planned at full capacity)
+  if (carry) {  // hints for the new lists; -1 = not known (planned somewhat above the largest recorded rank)
     m->rank_hint.assign(m->lists.farI.size(), -1);
     for (size_t q = 0; q < m->lists.farI.size(); q++) {
       const auto it = carried.find(((uint64_t)m->lists.farI[q] << 32) | (uint64_t)m->lists.farJ[q]);
@@ -509,11 +510,24 @@ std::vector<hignn::FarBlock> layout_batches(hignn_model* m, const std::vector<in
 // rank (batches of similar ranks need fewer iterations) and each batch runs its known
 // iteration count without reading counters back; a block that would need more terms than
 // recorded is deferred and rerun with the full capacity, so the result never depends on the
-// hint.
+// hint. A rebuild leaves most blocks without a rank (a split that moves by one particle shifts the ranges of
+// all nodes after it); these get the open capacity, a quarter and two terms above the largest rank last
+// recorded: the batch's iterations are as many, launched whether a block is left or not, and its pools as
+// large. (8,009 spheres at epsilon 1e-2, a rebuild every second step: largest ranks 20 to 29 from tree to
+// tree; 34 iterations instead of the full capacity's 100, four steps 31.2 instead of 35.4 ms. An
+// iteration with no block left takes about 15 us; a block that outgrows the capacity a rerun of its own, some
+// 20 iterations with read-backs, hence the margin.)
 // Pool capacity of a block without a recorded rank: about twice the largest rank of the
 // benchmark's far blocks at epsilon 1e-2 (14-18), so that the first far field on a tree packs up to
 // three times more blocks per batch than at the full capacity of max_iter = 100 terms.
 constexpr int kFirstPlanCap = 32;
+
+// After ranks were read back: their largest. Only the shard's own blocks have one.
+void record_hint_max(hignn_model* m) {
+  int r = 1;
+  for (int64_t q = m->sh_f0; q < m->sh_f1; q++) r = std::max(r, m->rank_hint[q]);
+  m->hint_max = std::min(r, m->max_iter);
+}
 
 void ensure_far_plan(hignn_model* m) {
   ensure_shard(m);
@@ -533,10 +547,11 @@ void ensure_far_plan(hignn_model* m) {
     full[q] = std::max(1, std::min(m->max_iter, std::min(nI, nJ)));
     idx[p] = (int)q;
   }
-  if (use_hints) {  // a block whose rank is not known (hint < 0) gets the full capacity
+  if (use_hints) {  // a block whose rank is not known (hint < 0) gets the open capacity
+    const int open = std::max(1, m->hint_max + m->hint_max / 4 + 2 + m->rank_hint_offset);
     std::vector<int> kc(m->lists.farI.size());
     for (int q : idx)
-      kc[q] = m->rank_hint[q] < 0 ? full[q] : std::max(1, std::min(full[q], m->rank_hint[q] + m->rank_hint_offset));
+      kc[q] = std::min(full[q], m->rank_hint[q] < 0 ? open : std::max(1, m->rank_hint[q] + m->rank_hint_offset));
     std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return kc[x] > kc[y]; });
     for (size_t p = 0; p < nf; p++) kcap[p] = kc[idx[p]];
   } else {
@@ -829,6 +844,7 @@ void far_field(hignn_model* m) {
     HIGNN_CUDA(cudaMemcpyAsync(m->rank_hint.data(), m->far_rank.p, sizeof(int32_t) * nf, cudaMemcpyDeviceToHost,
                                m->stream));
     HIGNN_CUDA(cudaStreamSynchronize(m->stream));
+    record_hint_max(m);
     m->hint_valid = true;
     m->hint_precision = m->precision;
     m->hint_epsilon = m->epsilon;
@@ -1142,6 +1158,7 @@ bool dot_graph(hignn_model* m, bool caller_order) {
                                  cudaMemcpyDeviceToHost, m->stream));
     }
     HIGNN_CUDA(cudaStreamSynchronize(m->stream));
+    if (!deferred.empty()) record_hint_max(m);
     if (m->precision >= 1) check_device_error(m);
   }
   m->stats.far_rank_sum = (int64_t)fst[0];
