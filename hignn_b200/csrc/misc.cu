@@ -41,23 +41,34 @@ __global__ void k_gather_positions(const float4* __restrict__ x4, const int32_t*
   out[i] = x4[pos[i]];
 }
 
+template <int Rows>
 __global__ void __launch_bounds__(simt::kThreads, simt::kCtasPerSm)
     k_eval_simt(const float* __restrict__ r, float* __restrict__ y, int64_t n, MlpF32 w) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   simt::Smem& s = *reinterpret_cast<simt::Smem*>(smem_raw);
+  constexpr int kTile = simt::kWarps * Rows;
   const int t = threadIdx.x;
   simt::load_weights(s, w);
-  for (int64_t base = (int64_t)blockIdx.x * simt::kTile; base < n; base += (int64_t)gridDim.x * simt::kTile) {
-    if (t < simt::kTile) {
+  for (int64_t base = (int64_t)blockIdx.x * kTile; base < n; base += (int64_t)gridDim.x * kTile) {
+    if (t < kTile) {
       const int64_t e = base + t;
       s.r[t] = e < n ? make_float4(r[3 * e], r[3 * e + 1], r[3 * e + 2], 0.f) : make_float4(1.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
-    simt::mlp_tile(s, w);
-    if (t < simt::kTile && base + t < n)
+    simt::mlp_tile<Rows>(s, w);
+    if (t < kTile && base + t < n)
 #pragma unroll
       for (int q = 0; q < 9; q++) y[9 * (base + t) + q] = s.y[t][q];
   }
+}
+
+template <int Rows>
+void eval_simt(const float* r, float* y, int64_t n, const MlpF32& w, int slots, cudaStream_t s) {
+  const size_t smem = sizeof(simt::Smem);
+  HIGNN_CUDA(cudaFuncSetAttribute(k_eval_simt<Rows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int64_t tiles = (n + simt::kWarps * Rows - 1) / (simt::kWarps * Rows);
+  k_eval_simt<Rows><<<(int)(tiles < slots ? tiles : slots), simt::kThreads, smem, s>>>(r, y, n, w);
+  HIGNN_CHECK_LAUNCH();
 }
 
 }  // namespace
@@ -82,12 +93,13 @@ void launch_gather_positions(const float4* x4, const int32_t* pos, float4* out, 
 
 void launch_eval_simt(const float* r, float* y, int64_t n, const MlpF32& w, int num_sms, cudaStream_t s) {
   if (n <= 0) return;
-  const size_t smem = sizeof(simt::Smem);
-  HIGNN_CUDA(cudaFuncSetAttribute(k_eval_simt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int64_t tiles = (n + simt::kTile - 1) / simt::kTile;
-  int grid = (int)(tiles < simt::kCtasPerSm * num_sms ? tiles : simt::kCtasPerSm * num_sms);
-  k_eval_simt<<<grid, simt::kThreads, smem, s>>>(r, y, n, w);
-  HIGNN_CHECK_LAUNCH();
+  const int slots = simt::kCtasPerSm * num_sms, rows = simt::rows_per_warp(n, slots);
+  if (rows == simt::kRows / 4)
+    eval_simt<simt::kRows / 4>(r, y, n, w, slots, s);
+  else if (rows == simt::kRows / 2)
+    eval_simt<simt::kRows / 2>(r, y, n, w, slots, s);
+  else
+    eval_simt<simt::kRows>(r, y, n, w, slots, s);
 }
 
 }  // namespace hignn

@@ -84,18 +84,30 @@ __device__ __forceinline__ void load_w2_slice(Smem& s, const MlpF32& w, int q) {
   cp_async_commit();
 }
 
-// Evaluates M(r) for s.r[0..63] (caller has written them and synchronized).
+// Evaluations per warp for n of them over `slots` CTAs: the smallest tile that takes them all at once. A
+// tile takes 65 us at 16 evaluations per warp, 43 at 8, 30 at 4 (92, 59 and 40 with two CTAs on the SM): the
+// weights and their slices cost the same for each. So fewer per warp is the better only
+// while it adds no second round (9,473 evaluations over 296 slots: 102 us at 8, 92 at 16).
+__host__ __device__ inline int rows_per_warp(int64_t n, int64_t slots) {
+  return n <= kTile / 4 * slots ? kRows / 4 : n <= kTile / 2 * slots ? kRows / 2 : kRows;
+}
+
+// Evaluates M(r) for s.r[0 .. kWarps * Rows - 1] (caller has written them and synchronized), Rows (16, 8 or 4) per
+// warp; the same operations in the same order per evaluation.
 // On return s.y[e][0..8] holds M row-major and the block is synchronized.
+template <int Rows = kRows>
 __device__ __forceinline__ void mlp_tile(Smem& s, const MlpF32& w) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, e0 = kRows * wid;
+  static_assert(Rows <= kRows && Rows % 4 == 0, "whole float4 of evaluations");
+  constexpr int kQuads = Rows / 4, kPairs = Rows / 2;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, e0 = Rows * wid;
   load_w2_slice(s, w, 0);
-  {  // layer 1 of the warp's evaluations: four of them and every eighth unit per thread
-    const int e = e0 + 4 * (lane & 3);
+  {  // layer 1 of the warp's evaluations: four of them and every 32 / kQuads-th unit per thread
+    const int e = e0 + 4 * (lane % kQuads);
     const float4 r0 = s.r[e], r1 = s.r[e + 1], r2 = s.r[e + 2], r3 = s.r[e + 3];
     const f2 x0 = f2_make(r0.x, r1.x), y0 = f2_make(r0.y, r1.y), z0 = f2_make(r0.z, r1.z);
     const f2 x1 = f2_make(r2.x, r3.x), y1 = f2_make(r2.y, r3.y), z1 = f2_make(r2.z, r3.z);
 #pragma unroll 2
-    for (int k = lane >> 2; k < kH1; k += 8) {
+    for (int k = lane / kQuads; k < kH1; k += 32 / kQuads) {
       const float4 c = s.w1b1[k];
       const f2 cx = f2_dup(c.x), cy = f2_dup(c.y), cz = f2_dup(c.z), cb = f2_dup(c.w);
       const f2 a = tanh_f32x2(f2_fma(cz, z0, f2_fma(cy, y0, f2_fma(cx, x0, cb))));
@@ -104,15 +116,15 @@ __device__ __forceinline__ void mlp_tile(Smem& s, const MlpF32& w) {
     }
     __syncwarp();
   }
-  // layer 3: lanes 0-23 take two evaluations (e3, e3 + 1 of the warp's) and three outputs (o3 ..) each
-  const int e3 = 2 * (lane & 7), o3 = lane < 24 ? 3 * (lane >> 3) : 0;
+  // layer 3: lanes 0 .. 3 kPairs - 1 take two evaluations (e3, e3 + 1 of the warp's) and three outputs (o3 ..) each
+  const int e3 = 2 * (lane % kPairs), o3 = lane < 3 * kPairs ? 3 * (lane / kPairs) : 0;
   f2 y3[3] = {f2_dup(0.f), f2_dup(0.f), f2_dup(0.f)};
   float(*h2)[kPieceStride] = s.h2[wid];
 #pragma unroll 1
   for (int c = 0; c < kH2 / kChunk; c++) {
-    f2 acc[kRows / 2][8];  // evaluation pairs x units lane + 32 j of the chunk
+    f2 acc[kPairs][8];  // evaluation pairs x units lane + 32 j of the chunk
 #pragma unroll
-    for (int i = 0; i < kRows / 2; i++)
+    for (int i = 0; i < kPairs; i++)
 #pragma unroll
       for (int j = 0; j < 8; j++) acc[i][j] = f2_dup(0.f);
 #pragma unroll 1
@@ -125,9 +137,9 @@ __device__ __forceinline__ void mlp_tile(Smem& s, const MlpF32& w) {
       const ulonglong2* hk = reinterpret_cast<const ulonglong2*>(&s.h1[q * kSlice][e0]);
 #pragma unroll 4
       for (int k = 0; k < kSlice; k++) {
-        f2 a[kRows / 2];
+        f2 a[kPairs];
 #pragma unroll
-        for (int i = 0; i < kRows / 4; i++) {
+        for (int i = 0; i < kQuads; i++) {
           const ulonglong2 v = hk[(size_t)k * (kTile / 4) + i];
           a[2 * i].v = v.x;
           a[2 * i + 1].v = v.y;
@@ -136,7 +148,7 @@ __device__ __forceinline__ void mlp_tile(Smem& s, const MlpF32& w) {
         for (int j = 0; j < 8; j++) {
           const f2 b = f2_dup(wk[k * kChunk + 32 * j]);
 #pragma unroll
-          for (int i = 0; i < kRows / 2; i++) acc[i][j] = f2_fma(a[i], b, acc[i][j]);
+          for (int i = 0; i < kPairs; i++) acc[i][j] = f2_fma(a[i], b, acc[i][j]);
         }
       }
     }
@@ -148,14 +160,14 @@ __device__ __forceinline__ void mlp_tile(Smem& s, const MlpF32& w) {
       for (int j = 0; j < 2; j++) {
         const f2 bias = f2_dup(s.b2[n0 + 32 * j + lane]);
 #pragma unroll
-        for (int i = 0; i < kRows / 4; i++)
+        for (int i = 0; i < kQuads; i++)
           *reinterpret_cast<ulonglong2*>(&h2[32 * j + lane][4 * i]) =
               make_ulonglong2(f2_add(acc[2 * i][2 * p + j], bias).v, f2_add(acc[2 * i + 1][2 * p + j], bias).v);
       }
       __syncwarp();
 #pragma unroll 2
-      for (int i = lane; i < kPiece * kRows / 4; i += 32) {  // tanh in place, four evaluations of a unit at a time
-        ulonglong2* v = reinterpret_cast<ulonglong2*>(&h2[i >> 2][4 * (i & 3)]);
+      for (int i = lane; i < kPiece * kQuads; i += 32) {  // tanh in place, four evaluations of a unit at a time
+        ulonglong2* v = reinterpret_cast<ulonglong2*>(&h2[i / kQuads][4 * (i % kQuads)]);
         const ulonglong2 x = *v;
         *v = make_ulonglong2(tanh_f32x2(f2{x.x}).v, tanh_f32x2(f2{x.y}).v);
       }
@@ -175,7 +187,7 @@ __device__ __forceinline__ void mlp_tile(Smem& s, const MlpF32& w) {
       }
     }
   }
-  if (lane < 24) {  // wrapper of python/convert.py:11-20: (y + b3 + I) / |r|, identity for |r| < 1e-5
+  if (lane < 3 * kPairs) {  // wrapper of python/convert.py:11-20: (y + b3 + I) / |r|, identity for |r| < 1e-5
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int e = e0 + e3 + q;
