@@ -970,7 +970,13 @@ uint64_t graph_signature(hignn_model* m) {
   mix((uint64_t)m->close_item0[m->sh_c0]);
   mix((uint64_t)m->close_item0[m->sh_c1]);
   mix((uint64_t)m->batches.size());
-  for (const auto& bt : m->batches) mix(((uint64_t)bt.b0 << 40) ^ ((uint64_t)bt.b1 << 16) ^ (uint64_t)bt.iters);
+  for (const auto& bt : m->batches) {
+    mix(((uint64_t)bt.b0 << 40) ^ ((uint64_t)bt.b1 << 16) ^ (uint64_t)bt.iters);
+    // the lengths of the batch's flag resets: another tree can have as many blocks in its batches
+    const auto& last = m->far_plan[bt.b1 - 1];
+    mix((uint64_t)last.rOff + last.nI);
+    mix((uint64_t)last.colOff + last.nJ);
+  }
   uint64_t e, t;
   std::memcpy(&e, &m->epsilon, 8);
   const double tol = std::max(m->student_tol, m->epsilon);
