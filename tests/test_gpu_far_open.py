@@ -54,3 +54,21 @@ def test_open_blocks_after_a_rebuild(precision, graph):
             # the second product at most: the open capacity, and a rerun of blocks above it
             assert m.stats()["far_iterations"] <= 2 * (top + top // 4 + 2) + 8
         m.close()
+
+
+def test_graph_over_rebuilds_of_like_shape():
+    """Small displacements leave the lists mostly as long as they were but shift the nodes' ranges: a captured
+    product must not be replayed on another tree's row counts."""
+    x = S.uniform(N, 0.1, 5)
+    f = S.sedimenting_forces(N, 5)
+    rng = np.random.default_rng(7)
+    m, e = make_model(x, 1), make_model(x, 1)
+    e.set(capi.P_GRAPH, 0)
+    for _ in range(8):
+        u, want = m.dot(f).astype(np.float64), e.dot(f).astype(np.float64)
+        assert np.linalg.norm(u - want) <= 1e-7 * np.linalg.norm(want)
+        x = (x + rng.normal(0, 0.01, x.shape)).astype(np.float32)
+        m.update_coord(x)
+        e.update_coord(x)
+    m.close()
+    e.close()
