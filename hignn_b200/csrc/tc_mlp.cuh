@@ -481,8 +481,12 @@ struct Epi {
     a1 = tl + kOffA1 + 32 * half;
     rows = tl + ((16 * half) << 16);
   }
+  // Whatever the warp does in tensor memory after a wait is ordered behind what the wait is for: the reading
+  // of an accumulator behind the MMAs that filled it, the writing of A1 and A2 behind those that read them.
   __device__ __forceinline__ bool wait(uint64_t* b, uint32_t parity, int code) {
-    return warp_wait(s, err, b, parity, code, prof);
+    const bool ok = warp_wait(s, err, b, parity, code, prof);
+    fence_after();
+    return ok;
   }
 
   // A1 <- tanh(W1 r + b1) of the warp's 32 rows and 64 hidden units as FP16 pairs (FP32 FMAs, bias
@@ -536,7 +540,6 @@ struct Epi {
   // Layer-3 accumulators of the warp's rows of tile t, complete, into shared memory. The server has
   // taken the outputs of tile t - 1: the features of t + 1, which it sent after that, are here.
   __device__ __forceinline__ void retire(uint32_t t) {
-    fence_after();
     uint32_t v[8];
     tmem_ld_frag16(rows + kOffD3 + 16 * (t & 1), v);
     tmem_wait_ld_of(v);
@@ -566,10 +569,8 @@ struct Epi {
         if (q == 3) {  // the last quarter is complete: every layer-2 MMA of this tile has read A1
           if (!wait(&s.feat_full[stream], (t + 1) & 1, 21)) return;
           have = t + 1 < *(volatile uint32_t*)&s.end_tile[stream];
-          fence_after();
           if (have) layer1(t + 1);
         }
-        fence_after();
         uint32_t v0[32], v1[32];
         tmem_ld_frag64(rows + kOffD2, v0);
         tmem_ld_frag64(rows + kOffD2 + 64, v1);
