@@ -1,4 +1,4 @@
-// The tanh of tanh_f32.cuh for two values at once, the same bit for bit, on the packed FP32 pipe.
+// The tanh of tanh_f32.cuh for two values at once, the same bit for bit (NaN for NaN), on the packed FP32 pipe.
 //
 // tanh_f32 branches between its two formulas, and a warp whose values fall on both sides of 0.8
 // runs both of them one value at a time (about 55 instructions). Here both are computed for a pair of values with
@@ -11,7 +11,8 @@
 //     by one Newton step on the hardware approximation, y + y (1 - d y): with a y that is good to an
 //     ulp and an exact fused residual the result is the correctly rounded reciprocal except where
 //     d's significand is all ones (Markstein, "Computation of elementary functions on the IBM RISC
-//     System/6000 processor", IBM J. Res. Dev. 34, 1990); checked against tanh_f32 for every finite input.
+//     System/6000 processor", IBM J. Res. Dev. 34, 1990); the tests compare the
+//     two functions for every input.
 #pragma once
 
 #include <cuda_runtime.h>
