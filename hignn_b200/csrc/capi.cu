@@ -19,7 +19,6 @@
 #include <fstream>
 #include <string>
 #include <thread>
-#include <unordered_map>
 #include <vector>
 
 #ifdef _OPENMP
@@ -134,7 +133,7 @@ struct hignn_model {
   // CUDA graph of the rank-planned H-matvec (HIGNN_P_GRAPH): captured once per plan and buffer
   // layout, replayed by every later product on the same tree and settings
   bool use_graph = true;
-  bool keep_ranks = true;  // HIGNN_P_KEEP_RANKS: ACA ranks carried across tree rebuilds
+  bool keep_ranks = true;  // HIGNN_P_KEEP_RANKS: the largest ACA rank is carried across tree rebuilds
   cudaGraphExec_t gexec = nullptr;       // near field (after the force gather)
   cudaGraphExec_t gexec_far = nullptr;   // far field (before the velocity scatter)
   uint64_t graph_sig = 0;
@@ -158,11 +157,15 @@ struct hignn_model {
   int plan_max_iter = -1;
   int64_t plan_rows = -1, plan_pool = -1;
   int plan_offset = 0;
-  // ACA ranks of the last far field (far-list order), valid for the same tree and settings
+  bool plan_open = false;    // blocks at the open capacity in the plan
+  bool plan_unread = false;  // ... and no product on it has told the ranks yet
+  int plan_exact = 0, plan_excess = 0, plan_spent = 0;  // iterations: see learn_ranks, spend_excess
+  // ACA ranks of the last far field (far-list order, -1 not known), valid for the same tree and settings
   std::vector<int32_t> rank_hint;
+  bool ranks_here = false;  // they are the ranks at the current positions
   bool hint_valid = false;
   int hint_precision = -1, hint_max_iter = -1;
-  int hint_max = 1;  // largest rank of this shard's blocks when ranks were last recorded; kept across rebuilds
+  int hint_max = 1;  // largest rank of this shard's blocks when ranks were last read back; kept across rebuilds
   double hint_epsilon = -1.0;
 
   hignn_stats stats{};
@@ -225,24 +228,11 @@ void cut_pair(hignn::PairWork w, int64_t per_item, std::vector<hignn::PairWork>&
 // later call runs on lists that do not belong to the uploaded positions.
 void build_structures(hignn_model* m) {
   const auto t0 = std::chrono::steady_clock::now();
-  // ACA ranks of the previous far field, keyed by the two nodes of each block (ids and particle
-  // ranges): a block of the new lists that joins the same two nodes starts from that rank
-  struct Carried {
-    int64_t sI, eI, sJ, eJ;
-    int32_t rank;
-  };
-  std::unordered_map<uint64_t, Carried> carried;
-  const bool carry = m->keep_ranks && m->hint_valid && m->rank_hint.size() == m->lists.farI.size() && m->tree_ready;
-  if (carry)
-    for (size_t q = 0; q < m->lists.farI.size(); q++) {
-      const auto& I = m->tree.nodes[m->lists.farI[q]];
-      const auto& J = m->tree.nodes[m->lists.farJ[q]];
-      carried[((uint64_t)m->lists.farI[q] << 32) | (uint64_t)m->lists.farJ[q]] =
-          Carried{I.start, I.end, J.start, J.end, m->rank_hint[q]};
-    }
+  const bool carry = m->keep_ranks && m->hint_valid && m->tree_ready;
   m->tree_ready = false;
   m->plan_ready = false;
   m->hint_valid = false;
+  m->ranks_here = false;
   m->shard_ready = false;
   const bool on_dev = m->device >= 0 && m->tree_on_device;
   hignn::ClusterTree tree;
@@ -285,16 +275,8 @@ void build_structures(hignn_model* m) {
   m->lists = std::move(lists);
   m->lists_sym = m->use_symmetry;
   m->lists_max_rel = m->max_relative_coord;
-  if (carry) {  // hints for the new lists; -1 = not known (planned somewhat above the largest recorded rank)
+  if (carry) {  // the new blocks have no ranks of their own; hint_max stays
     m->rank_hint.assign(m->lists.farI.size(), -1);
-    for (size_t q = 0; q < m->lists.farI.size(); q++) {
-      const auto it = carried.find(((uint64_t)m->lists.farI[q] << 32) | (uint64_t)m->lists.farJ[q]);
-      if (it == carried.end()) continue;
-      const auto& I = m->tree.nodes[m->lists.farI[q]];
-      const auto& J = m->tree.nodes[m->lists.farJ[q]];
-      const Carried& c = it->second;
-      if (c.sI == I.start && c.eI == I.end && c.sJ == J.start && c.eJ == J.end) m->rank_hint[q] = c.rank;
-    }
     m->hint_valid = true;
   }
   const auto t1 = std::chrono::steady_clock::now();
@@ -425,6 +407,14 @@ bool hints_usable(const hignn_model* m) {
          m->hint_max_iter == m->max_iter && m->rank_hint.size() == m->lists.farI.size();
 }
 
+// A pool of at least `bytes`. One that is too small grows with a quarter to spare, as far as the budget of a
+// batch allows: the largest rank, and with it the pools, differs from tree to tree (giving back and allocating
+// some GB takes tens to hundreds of milliseconds).
+void ensure_pool(const hignn_model* m, DevBuf& pool, size_t bytes) {
+  if (pool.p && pool.bytes < bytes) bytes = std::max(bytes, std::min(bytes + bytes / 4, (size_t)m->far_pool_bytes / 2));
+  pool.ensure(bytes);
+}
+
 // Lays out far blocks `idx` (far-list positions) with pool capacities `kcap` into ACA batches:
 // a batch is cut when its C + Q pools (9 doubles per particle and term) would exceed
 // far_pool_bytes or its rows (sum of |I| + |J|) far_batch_rows. Grows the device buffers to
@@ -489,8 +479,8 @@ std::vector<hignn::FarBlock> layout_batches(hignn_model* m, const std::vector<in
     m->far_cols.ensure(sizeof(int32_t) * (size_t)maxNb * ldr);
     m->far_used_row.ensure((size_t)maxR + 16);
     m->far_used_col.ensure((size_t)maxCol + 16);
-    m->far_C.ensure(sizeof(hignn::pool_t) * 9 * (size_t)maxC);
-    m->far_Q.ensure(sizeof(hignn::pool_t) * 9 * (size_t)maxQ);
+    ensure_pool(m, m->far_C, sizeof(hignn::pool_t) * 9 * (size_t)maxC);
+    ensure_pool(m, m->far_Q, sizeof(hignn::pool_t) * 9 * (size_t)maxQ);
     m->far_xc.ensure(sizeof(float) * (size_t)maxX);
     m->far_act.ensure(sizeof(int32_t) * (maxNb + 1));
     m->far_preI.ensure(sizeof(int32_t) * (maxNb + 1));
@@ -505,28 +495,79 @@ std::vector<hignn::FarBlock> layout_batches(hignn_model* m, const std::vector<in
 // ACA plan of the far list. Without rank information every block gets the pool capacity
 // min(max_iter, |I|, |J|, kFirstPlanCap) and the batches follow the list order
 // (src/FarDot.cpp:191-340 batches the list in order); a block that needs more terms is deferred
-// and rerun with min(max_iter, |I|, |J|), so the cap only decides how many blocks share a batch. When the previous far field on the same tree and settings
-// recorded every block's rank, each block gets exactly that capacity, the blocks are sorted by
-// rank (batches of similar ranks need fewer iterations) and each batch runs its known
-// iteration count without reading counters back; a block that would need more terms than
-// recorded is deferred and rerun with the full capacity, so the result never depends on the
-// hint. A rebuild leaves most blocks without a rank (a split that moves by one particle shifts the ranges of
-// all nodes after it); these get the open capacity, a quarter and two terms above the largest rank last
-// recorded: the batch's iterations are as many, launched whether a block is left or not, and its pools as
-// large. (8,009 spheres at epsilon 1e-2, a rebuild every second step: largest ranks 20 to 29 from tree to
-// tree; 34 iterations instead of the full capacity's 100, four steps 31.2 instead of 35.4 ms. An
-// iteration with no block left takes about 15 us; a block that outgrows the capacity a rerun of its own, some
-// 20 iterations with read-backs, hence the margin.)
+// and rerun with min(max_iter, |I|, |J|), so the cap only decides how many blocks share a batch. Once a far field with
+// these settings has told the ranks, each batch runs a known iteration count without reading counters back:
+//   * at the positions the ranks belong to, a block's capacity is its rank, and the blocks are sorted by it (batches of
+//     similar ranks need fewer iterations);
+//   * where the positions have moved since, or the tree was rebuilt, every block has the open capacity. The rank
+//     of one block is no guide there: displacements of 0.005 radii move it by several terms either way,
+//     and a few blocks above their capacity cost a rerun of some 20 iterations with read-backs. (One B200, epsilon 1e-2,
+//     products on one tree after displacements of 0.005, median: with the ranks and a quarter and two terms / with
+//     the open capacity, 8,009 uniform spheres 8.9 / 5.9 ms, 32,768 37.4 / 32.3 ms, 131,072 189 / 169 ms. The full
+//     capacity instead of the open one costs its empty iterations, about 15 us each, and three times the pools.)
+// A block that would need more terms than its capacity is deferred and rerun with the full one, so the result depends
+// on the hints only as far as the order in which a block's stopping norms are summed does (it follows the number of
+// blocks in a batch, far_aca.cu).
 // Pool capacity of a block without a recorded rank: about twice the largest rank of the
 // benchmark's far blocks at epsilon 1e-2 (14-18), so that the first far field on a tree packs up to
 // three times more blocks per batch than at the full capacity of max_iter = 100 terms.
 constexpr int kFirstPlanCap = 32;
 
-// After ranks were read back: their largest. Only the shard's own blocks have one.
-void record_hint_max(hignn_model* m) {
-  int r = 1;
-  for (int64_t q = m->sh_f0; q < m->sh_f1; q++) r = std::max(r, m->rank_hint[q]);
-  m->hint_max = std::min(r, m->max_iter);
+// The open capacity: a quarter and two terms above the largest rank of the last far field whose ranks were read.
+int open_capacity(const hignn_model* m) { return m->hint_max + m->hint_max / 4 + 2; }
+
+// Copies the ranks of the far field just run to the host (the caller synchronises before learn_ranks). Before
+// any rerun by the teacher, so that a block sent back to it keeps the rank of the student's queries, which the plan
+// is for.
+void fetch_ranks(hignn_model* m, std::vector<int32_t>& ranks) {
+  ranks.resize(m->lists.farI.size());
+  HIGNN_CUDA(cudaMemcpyAsync(ranks.data(), m->far_rank.p, sizeof(int32_t) * ranks.size(), cudaMemcpyDeviceToHost,
+                             m->stream));
+}
+
+// The hints of the next plan from the ranks of a far field whose blocks `deferred` outgrew the current plan. The
+// plan is dropped when some did and their capacities change: left as it is, every product on the tree would
+// defer and rerun them (8,009 spheres drawn together on their tree: 6.4 ms for each product with the plan kept, 4.9 ms
+// with it made again, which takes 0.1 to 0.8 ms once). Otherwise it
+// is kept, and plan_excess tells how many iterations a product on it runs beyond what the ranks need.
+void learn_ranks(hignn_model* m, const std::vector<int32_t>& ranks, const std::vector<int>& deferred) {
+  const size_t nf = m->lists.farI.size();
+  if (!m->plan_hinted || m->rank_hint.size() != nf) m->rank_hint.assign(nf, -1);
+  std::vector<int32_t> hint = m->rank_hint;
+  int top = 1;
+  for (int64_t q = m->sh_f0; q < m->sh_f1; q++) top = std::max(top, hint[q] = ranks[q]);
+  if (!deferred.empty()) {
+    // a deferred block gets a larger capacity than it had, whatever rank its rerun gave: the width of the pivot
+    // CTAs follows the number of blocks in a batch, and the stopping norms their order of summation
+    std::vector<int> cap(nf, 0);
+    for (const auto& fb : m->far_plan) cap[fb.list_idx] = fb.kcap;
+    for (int q : deferred) hint[q] = std::max(hint[q], cap[q] + 1);
+    if (hint != m->rank_hint) m->plan_ready = false;
+  }
+  m->rank_hint = std::move(hint);
+  m->hint_max = std::min(top, m->max_iter);
+  m->hint_valid = true;
+  m->ranks_here = true;
+  m->hint_precision = m->precision;
+  m->hint_epsilon = m->epsilon;
+  m->hint_max_iter = m->max_iter;
+  m->plan_unread = false;
+  m->plan_exact = m->plan_excess = m->plan_spent = 0;
+  for (const auto& bt : m->batches) {
+    int need = 1;
+    for (int b = bt.b0; b < bt.b1; b++) need = std::max(need, m->rank_hint[m->far_plan[b].list_idx]);
+    m->plan_exact += need;
+    m->plan_excess += std::max(0, bt.iters - need);
+  }
+}
+
+// After a product whose ranks were known: the plan is made again, from them and without a margin, once the iterations
+// that products at these positions ran in excess are as many as it has iterations itself. (An iteration with no
+// block left takes about 15 us; planning and capturing again takes about as much for each of the plan's.)
+void spend_excess(hignn_model* m) {
+  if (!m->ranks_here || !m->plan_open) return;
+  m->plan_spent += m->plan_excess;
+  if (m->plan_excess > 0 && m->plan_spent >= m->plan_exact) m->plan_ready = false;
 }
 
 void ensure_far_plan(hignn_model* m) {
@@ -534,7 +575,7 @@ void ensure_far_plan(hignn_model* m) {
   const bool use_hints = hints_usable(m);
   if (m->plan_ready && m->plan_hinted == use_hints && m->plan_max_iter == m->max_iter &&
       m->plan_rows == m->far_batch_rows && m->plan_pool == m->far_pool_bytes &&
-      m->plan_offset == m->rank_hint_offset)
+      m->plan_offset == m->rank_hint_offset && (!use_hints || m->plan_open || m->ranks_here))
     return;
   const size_t nf = (size_t)(m->sh_f1 - m->sh_f0);
   std::vector<int> idx(nf), kcap(nf);
@@ -547,11 +588,14 @@ void ensure_far_plan(hignn_model* m) {
     full[q] = std::max(1, std::min(m->max_iter, std::min(nI, nJ)));
     idx[p] = (int)q;
   }
-  if (use_hints) {  // a block whose rank is not known (hint < 0) gets the open capacity
-    const int open = std::max(1, m->hint_max + m->hint_max / 4 + 2 + m->rank_hint_offset);
+  m->plan_open = false;
+  if (use_hints) {
     std::vector<int> kc(m->lists.farI.size());
-    for (int q : idx)
-      kc[q] = std::min(full[q], m->rank_hint[q] < 0 ? open : std::max(1, m->rank_hint[q] + m->rank_hint_offset));
+    for (int q : idx) {
+      const bool known = m->ranks_here && m->rank_hint[q] >= 0;
+      m->plan_open |= !known;
+      kc[q] = std::min(full[q], std::max(1, (known ? m->rank_hint[q] : open_capacity(m)) + m->rank_hint_offset));
+    }
     std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return kc[x] > kc[y]; });
     for (size_t p = 0; p < nf; p++) kcap[p] = kc[idx[p]];
   } else {
@@ -566,6 +610,8 @@ void ensure_far_plan(hignn_model* m) {
   }
   m->plan_ready = true;
   m->plan_hinted = use_hints;
+  m->plan_unread = m->plan_open;
+  m->plan_exact = m->plan_excess = m->plan_spent = 0;
   m->plan_max_iter = m->max_iter;
   m->plan_rows = m->far_batch_rows;
   m->plan_pool = m->far_pool_bytes;
@@ -823,6 +869,9 @@ void far_field(hignn_model* m) {
     if (!r2.deferred.empty()) throw Error(HIGNN_ERR_LIMIT, "ACA: a block was deferred at its full capacity");
     fallback.insert(fallback.end(), r2.fallback.begin(), r2.fallback.end());
   }
+  const bool learn = !m->plan_hinted || m->plan_unread || had_deferred;
+  std::vector<int32_t> ranks;
+  if (learn) fetch_ranks(m, ranks);
   if (!fallback.empty()) {  // student residual above tolerance: the teacher network for these blocks
     FarOutcome r3;
     run_far_subset(m, fallback, false, &iterations, &r3);
@@ -839,17 +888,10 @@ void far_field(hignn_model* m) {
   m->stats.t_far_active_ms = m->far_timer.active_ms;
   // per ACA iteration: active list, column eval, column pivot, row eval, row pivot
   m->stats.gpu_launches += 5 * (int64_t)iterations;
-  if (!m->plan_hinted || had_deferred) {  // record the ranks for the next far field on this tree
-    m->rank_hint.resize(nf);
-    HIGNN_CUDA(cudaMemcpyAsync(m->rank_hint.data(), m->far_rank.p, sizeof(int32_t) * nf, cudaMemcpyDeviceToHost,
-                               m->stream));
-    HIGNN_CUDA(cudaStreamSynchronize(m->stream));
-    record_hint_max(m);
-    m->hint_valid = true;
-    m->hint_precision = m->precision;
-    m->hint_epsilon = m->epsilon;
-    m->hint_max_iter = m->max_iter;
-  }
+  if (learn)
+    learn_ranks(m, ranks, res.deferred);
+  else
+    spend_excess(m);
 }
 
 void near_field(hignn_model* m) {
@@ -915,6 +957,7 @@ void refit_positions(hignn_model* m) {
     m->xt[3 * i + 2] = m->xyz[3 * p + 2];
     x4[i] = make_float4(m->xt[3 * i], m->xt[3 * i + 1], m->xt[3 * i + 2], 0.f);
   }
+  m->ranks_here = false;
   if (m->device < 0) return;
   HIGNN_CUDA(cudaMemcpyAsync(m->x4.p, x4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, m->stream));
   HIGNN_CUDA(cudaStreamSynchronize(m->stream));
@@ -1105,7 +1148,9 @@ bool dot_graph(hignn_model* m, bool caller_order) {
   unsigned long long fst[2] = {0, 0};
   int err = 0;
   const bool far_on = (m->fields & 2) && !m->batches.empty();
+  std::vector<int32_t> ranks;
   if (far_on) {
+    if (m->plan_unread) fetch_ranks(m, ranks);
     HIGNN_CUDA(cudaMemcpyAsync(status, m->far_status.p, sizeof(status), cudaMemcpyDeviceToHost, m->stream));
     HIGNN_CUDA(cudaMemcpyAsync(fst, m->far_stats.p, sizeof(fst), cudaMemcpyDeviceToHost, m->stream));
   }
@@ -1129,13 +1174,14 @@ bool dot_graph(hignn_model* m, bool caller_order) {
     m->stats.t_far_ms = b;
     m->stats.t_dot_ms = a + b;
   }
+  std::vector<int> deferred;
   if (far_on && (status[0] > 0 || status[1] > 0)) {  // reruns, eagerly, then the scatter again
     const int cap = (int)nf;
     std::vector<int32_t> lists(2 * (size_t)cap);
     HIGNN_CUDA(cudaMemcpyAsync(lists.data(), m->far_status.as<int>() + 8, sizeof(int32_t) * 2 * cap,
                                cudaMemcpyDeviceToHost, m->stream));
     HIGNN_CUDA(cudaStreamSynchronize(m->stream));
-    std::vector<int> deferred(lists.begin(), lists.begin() + std::min(status[0], cap));
+    deferred.assign(lists.begin(), lists.begin() + std::min(status[0], cap));
     std::vector<int> fallback(lists.begin() + cap, lists.begin() + cap + std::min(status[1], cap));
     std::sort(deferred.begin(), deferred.end());
     std::sort(fallback.begin(), fallback.end());
@@ -1146,6 +1192,7 @@ bool dot_graph(hignn_model* m, bool caller_order) {
       run_far_subset(m, deferred, student_pass, &iters, &r2);
       if (!r2.deferred.empty()) throw Error(HIGNN_ERR_LIMIT, "ACA: a block was deferred at its full capacity");
       fallback.insert(fallback.end(), r2.fallback.begin(), r2.fallback.end());
+      fetch_ranks(m, ranks);
     }
     if (!fallback.empty()) {
       FarOutcome r3;
@@ -1158,15 +1205,13 @@ bool dot_graph(hignn_model* m, bool caller_order) {
       hignn::launch_scatter_velocities(m->u.as<double>(), m->perm.as<int32_t>(), m->io_u.as<float>(), m->n,
                                        m->stream);
     HIGNN_CUDA(cudaMemcpyAsync(fst, m->far_stats.p, sizeof(fst), cudaMemcpyDeviceToHost, m->stream));
-    if (!deferred.empty()) {  // ranks recorded again for the next plan
-      m->rank_hint.resize(m->lists.farI.size());
-      HIGNN_CUDA(cudaMemcpyAsync(m->rank_hint.data(), m->far_rank.p, sizeof(int32_t) * m->rank_hint.size(),
-                                 cudaMemcpyDeviceToHost, m->stream));
-    }
     HIGNN_CUDA(cudaStreamSynchronize(m->stream));
-    if (!deferred.empty()) record_hint_max(m);
     if (m->precision >= 1) check_device_error(m);
   }
+  if (!ranks.empty())
+    learn_ranks(m, ranks, deferred);
+  else if (far_on)
+    spend_excess(m);
   m->stats.far_rank_sum = (int64_t)fst[0];
   m->stats.far_evals = (int64_t)fst[1];
   return true;
@@ -1620,6 +1665,7 @@ void tb_add_device(hignn_tb* t, hignn_model* m);
 // terms when a three-body object is attached.
 void step_velocity(hignn_model* m, const hignn_force_model& fm) {
   const int64_t n = m->n;
+  m->ranks_here = false;  // the loops move the positions between any two evaluations
   HIGNN_CUDA(cudaEventRecord(m->lev[0], m->stream));
   apply_forces(m, m->x4.as<float4>(), n, m->slot.as<int32_t>(), fm, m->f4.as<float4>(), nullptr);
   HIGNN_CUDA(cudaMemsetAsync(m->u.p, 0, sizeof(double) * 3 * n, m->stream));
@@ -1628,6 +1674,7 @@ void step_velocity(hignn_model* m, const hignn_force_model& fm) {
     matvec_tree_order(m);
     m->loop_prof[7] += 1;
   }
+  m->ranks_here = false;
   HIGNN_CUDA(cudaEventRecord(m->lev[2], m->stream));
   if (m->tb) tb_add_device(m->tb, m);
   HIGNN_CUDA(cudaEventRecord(m->lev[3], m->stream));
