@@ -149,6 +149,8 @@ struct hignn_model {
   // far-field plan: blocks in batch order; iters > 0 when every block's rank is known
   struct Batch {
     int b0, b1, iters;
+    int mean_rows, max_rows;  // of its blocks
+    std::vector<int> active;  // known iterations: blocks expected to be left in each
   };
   std::vector<hignn::FarBlock> far_plan;
   std::vector<Batch> batches;
@@ -163,6 +165,7 @@ struct hignn_model {
   // ACA ranks of the last far field (far-list order, -1 not known), valid for the same tree and settings
   std::vector<int32_t> rank_hint;
   bool ranks_here = false;  // they are the ranks at the current positions
+  std::vector<float> rank_share;  // share of the blocks with a rank above k when ranks were last read back
   bool hint_valid = false;
   int hint_precision = -1, hint_max_iter = -1;
   int hint_max = 1;  // largest rank of this shard's blocks when ranks were last read back; kept across rebuilds
@@ -425,7 +428,22 @@ std::vector<hignn::FarBlock> layout_batches(hignn_model* m, const std::vector<in
   batches.clear();
   int64_t rows = 0, cE = 0, qE = 0, xE = 0, maxC = 0, maxQ = 0, maxX = 0;
   int32_t rOff = 0, colOff = 0, maxR = 0, maxCol = 0;
-  int b0 = 0, maxNb = 0, iters = 0;
+  int b0 = 0, maxNb = 0, iters = 0, largest = 0;
+  auto close_batch = [&](int b1) {
+    hignn_model::Batch bt{b0, b1, known ? iters : 0, (int)(rows / (2 * (b1 - b0))), largest, {}};
+    if (known) {
+      bt.active.assign(iters, 0);
+      if (m->plan_open)
+        for (int k = 0; k < iters; k++)
+          bt.active[k] = k < (int)m->rank_share.size() ? (int)std::ceil(m->rank_share[k] * (b1 - b0)) : 0;
+      else
+        for (int p = b0; p < b1; p++) bt.active[kcap[p] - 1]++;
+      if (!m->plan_open)
+        for (int k = iters - 2; k >= 0; k--) bt.active[k] += bt.active[k + 1];
+    }
+    batches.push_back(std::move(bt));
+    maxNb = std::max(maxNb, b1 - b0);
+  };
   for (size_t p = 0; p < idx.size(); p++) {
     const int q = idx[p];
     const auto& I = m->tree.nodes[m->lists.farI[q]];
@@ -435,12 +453,11 @@ std::vector<hignn::FarBlock> layout_batches(hignn_model* m, const std::vector<in
     const int64_t add = (int64_t)kcap[p] * (nI + nJ) * 9 * (int64_t)sizeof(hignn::pool_t);
     if (cnt > 0 && ((cE + qE) * 9 * (int64_t)sizeof(hignn::pool_t) + add > m->far_pool_bytes ||
                     rows + nI + nJ > m->far_batch_rows)) {
-      batches.push_back({b0, (int)p, known ? iters : 0});
-      maxNb = std::max(maxNb, cnt);
+      close_batch((int)p);
       b0 = (int)p;
       rows = cE = qE = xE = 0;
       rOff = colOff = 0;
-      iters = 0;
+      iters = largest = 0;
     }
     hignn::FarBlock fb{};
     fb.sI = (int32_t)I.start;
@@ -461,6 +478,7 @@ std::vector<hignn::FarBlock> layout_batches(hignn_model* m, const std::vector<in
     colOff += nJ;
     rows += nI + nJ;
     iters = std::max(iters, fb.kcap);
+    largest = std::max(largest, (int)std::max(nI, nJ));
     maxC = std::max(maxC, cE);
     maxQ = std::max(maxQ, qE);
     maxX = std::max(maxX, xE);
@@ -468,10 +486,7 @@ std::vector<hignn::FarBlock> layout_batches(hignn_model* m, const std::vector<in
     maxCol = std::max(maxCol, colOff);
     out[p] = fb;
   }
-  if (!idx.empty()) {
-    batches.push_back({b0, (int)idx.size(), known ? iters : 0});
-    maxNb = std::max(maxNb, (int)idx.size() - b0);
-  }
+  if (!idx.empty()) close_batch((int)idx.size());
   if (m->device >= 0 && !idx.empty()) {
     const int ldr = m->max_iter + 1;
     m->far_state.ensure(sizeof(hignn::FarState) * maxNb);
@@ -543,6 +558,14 @@ void learn_ranks(hignn_model* m, const std::vector<int32_t>& ranks, const std::v
     for (const auto& fb : m->far_plan) cap[fb.list_idx] = fb.kcap;
     for (int q : deferred) hint[q] = std::max(hint[q], cap[q] + 1);
     if (hint != m->rank_hint) m->plan_ready = false;
+  }
+  m->rank_share.assign(top, 0.f);
+  int64_t above = m->sh_f1 - m->sh_f0;
+  std::vector<int64_t> ending(top + 1, 0);
+  for (int64_t q = m->sh_f0; q < m->sh_f1; q++) ending[std::max(0, ranks[q])]++;
+  for (int k = 0; k < top; k++) {
+    above -= ending[k];
+    m->rank_share[k] = (float)((double)above / (double)(m->sh_f1 - m->sh_f0));
   }
   m->rank_hint = std::move(hint);
   m->hint_max = std::min(top, m->max_iter);
@@ -748,6 +771,8 @@ hignn::FarArgs far_args(hignn_model* m, const hignn_model::Batch& bt, const hign
   a.use_symmetry = m->use_symmetry ? 1 : 0;
   a.defer_apply = student_pass ? 1 : 0;
   a.fast_pivots = m->precision >= 1 ? 1 : 0;
+  a.mean_rows = bt.mean_rows;
+  a.max_rows = bt.max_rows;
   return a;
 }
 
@@ -766,7 +791,7 @@ FarOutcome run_far_batches(hignn_model* m, const std::vector<hignn::FarBlock>& p
     HIGNN_CUDA(cudaMemsetAsync(m->far_used_col.p, 0, (size_t)last.colOff + last.nJ, m->stream));
     hignn::FarTimer* tm = m->timing >= 2 ? &m->far_timer : nullptr;
     const int nd = hignn::far_batch_plain(a, w, m->precision >= 1 ? &tcw : nullptr, student, m->err_flag(),
-                                          m->num_sms, m->host_ctr, m->stream, bt.iters, iterations, tm);
+                                          m->num_sms, m->host_ctr, m->stream, bt.iters, bt.active, iterations, tm);
     m->stats.far_rank_max = std::max(m->stats.far_rank_max, m->host_ctr[hignn::kCtrRankMax]);
     m->stats.gpu_launches += 1;
     const int nb = bt.b1 - bt.b0, ld = a.ldr;
@@ -1015,6 +1040,10 @@ uint64_t graph_signature(hignn_model* m) {
   mix((uint64_t)m->batches.size());
   for (const auto& bt : m->batches) {
     mix(((uint64_t)bt.b0 << 40) ^ ((uint64_t)bt.b1 << 16) ^ (uint64_t)bt.iters);
+    const hignn::FarArgs a = far_args(m, bt, nullptr, false);
+    uint64_t widths = 0;
+    for (int k = 0; k < (int)bt.active.size(); k++)
+      mix(widths = 5 * widths + (uint64_t)hignn::far_pivot_width(a, k, bt.active[k], m->num_sms));
     // the lengths of the batch's flag resets: another tree can have as many blocks in its batches
     const auto& last = m->far_plan[bt.b1 - 1];
     mix((uint64_t)last.rOff + last.nI);
@@ -1065,7 +1094,7 @@ void graph_far_body(hignn_model* m, bool caller_order) {
       HIGNN_CUDA(cudaMemsetAsync(m->far_used_row.p, 0, (size_t)last.rOff + last.nI, m->stream));
       HIGNN_CUDA(cudaMemsetAsync(m->far_used_col.p, 0, (size_t)last.colOff + last.nJ, m->stream));
       hignn::far_batch_launch(a, w, m->precision >= 1 ? &tcw : nullptr, student, m->err_flag(), m->num_sms,
-                              m->stream, bt.iters);
+                              m->stream, bt.iters, bt.active);
       if (student_pass) {
         const size_t ns = (size_t)a.nb * hignn::kFarSamples;
         float* feat = m->far_check.as<float>();

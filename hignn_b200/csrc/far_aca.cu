@@ -35,15 +35,22 @@ constexpr int kPivThreads = 128;
 // slower at N = 1M (287 ms of pivots at 8, 297 at 10, 315 at 12, 337 for the FP64 form)
 constexpr int kPivBlocksF32 = 8;
 constexpr int kApplyThreads = 256;  // the deferred apply: few phases, wider CTAs
-// Where a batch has few blocks, an iteration lasts as long as its largest block: the same kernels then run
-// 512-thread CTAs (the orthogonalisation takes four chunks at once, the cross terms sixteen l). Measured,
-// column + row pivots of one product, 128 against 512 threads: 365 blocks (4,096 spheres, epsilon 1e-5, 100
-// iterations, FP64) 5.8 + 22.9 against 4.3 + 13.8 ms; 750 blocks (5,003 spheres, 1e-2, FP32) 0.48 + 1.01 against
-// 0.49 + 0.89; 1,151 blocks (four products) 2.7 + 5.5 against 3.2 + 4.8; 3,072 blocks (12,289 spheres, FP64)
-// 0.93 + 3.10 against 1.20 + 3.11; 13,453 blocks 3.2 + 5.0 against 4.6 + 6.3. Hence the two lines, in blocks per SM.
+// Where few blocks are left, an iteration lasts as long as its largest block: the same kernels then run
+// 512-thread CTAs (the orthogonalisation takes four chunks at once, the cross terms sixteen l). Two of them share an
+// SM, against eight of the narrow ones, so the rule follows the blocks expected to be left. Measured per launch (us, 128
+// against 512 threads; col and row pivot):
+//   5,003 spheres, FP32: 777 blocks left 16 / 27 and 16 / 29, 361: 22 / 25 and 41 / 39, 207: 23 / 18 and 47 / 31,
+//     17: 24 / 18 and 60 / 41; at 1e-4, iteration 60, 759 blocks 138 / 156 and 192 / 297, iteration 84, 121 blocks 139 / 76
+//     and 167 / 135. FP64: 777 blocks, iteration 36, 58 / 89 and 176 / 211, 119 blocks, iteration 84, 94 / 57 and 291 / 174.
+//   2,003 spheres in leaves of 32 (34 rows per block on average): 320 blocks left 15 / 23 and 25 / 35, 25: 17 / 16 and 35 / 29;
+//     700 in leaves of 16 (14 rows): 118 blocks 12 / 13 and 20 / 23. Small blocks have nothing to share out.
+//   Row pivots of batches with blocks above 256 rows (three chunks and more for a narrow CTA): FP32 8,009 spheres, 628
+//     blocks 57 / 53, 698 (separated) 80 / 58; FP64 8,009 spheres, 1,073 blocks, iteration 36, 363 / 305, 760 blocks, iteration
+//     96, 900 / 629; 6,000 clustered spheres, 623 blocks, iteration 24, 217 / 137. In the first iterations they lose as well.
 constexpr int kWideThreads = 512;
 constexpr int kWideBlocks = 2;
-constexpr int kWideColLimit = 4, kWideRowLimit = 8;
+constexpr int kWideMeanRows = 48, kWideLargeRows = 256;
+
 
 template <typename T>
 __device__ __forceinline__ T det3(const T* m) {
@@ -1040,7 +1047,7 @@ namespace {
 // One ACA iteration of every active block of a batch: active list, column queries, column pivot,
 // row queries, row pivot (with the stop test and, unless deferred, the apply).
 void far_iteration(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, const float* student, int* err,
-                   int num_sms, cudaStream_t s, FarTimer* timer) {
+                   int num_sms, cudaStream_t s, FarTimer* timer, int k, int left) {
   auto mark = [&]() {
     if (timer) HIGNN_CUDA(cudaEventRecord(timer->next(), s));
   };
@@ -1048,7 +1055,9 @@ void far_iteration(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, cons
   const size_t row_smem = sizeof(double) * (9 + 3 + 3) * a.ldr;
   const size_t col_smem = sizeof(double) * 9 * a.ldr;
   const int piv_grid = a.nb < 16 * num_sms ? a.nb : 16 * num_sms;  // grid-stride over active blocks
-  const bool wide_col = a.nb <= kWideColLimit * num_sms, wide_row = a.nb <= kWideRowLimit * num_sms;
+  const int wide_grid = a.nb < 8 * num_sms ? a.nb : 8 * num_sms;
+  const int width = far_pivot_width(a, k, left, num_sms);
+  const bool wide_col = (width & 1) != 0, wide_row = (width & 2) != 0;
   mark();
   k_far_active<<<1, 1024, 0, s>>>(a);
   mark();
@@ -1060,11 +1069,11 @@ void far_iteration(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, cons
     k_far_eval<<<simt::kCtasPerSm * num_sms, simt::kThreads, eval_smem, s>>>(a, w, 0);
   mark();
   if (a.fast_pivots && wide_col)
-    k_far_col_pivot_f32<kWideThreads, kWideBlocks><<<a.nb, kWideThreads, col_smem_f32(a.ldr, kWideThreads), s>>>(a);
+    k_far_col_pivot_f32<kWideThreads, kWideBlocks><<<wide_grid, kWideThreads, col_smem_f32(a.ldr, kWideThreads), s>>>(a);
   else if (a.fast_pivots)
     k_far_col_pivot_f32<kPivThreads, kPivBlocksF32><<<piv_grid, kPivThreads, col_smem_f32(a.ldr, kPivThreads), s>>>(a);
   else if (wide_col)
-    k_far_col_pivot<double, kWideThreads, kWideBlocks><<<a.nb, kWideThreads, col_smem, s>>>(a);
+    k_far_col_pivot<double, kWideThreads, kWideBlocks><<<wide_grid, kWideThreads, col_smem, s>>>(a);
   else
     k_far_col_pivot<double, kPivThreads, 8><<<piv_grid, kPivThreads, col_smem, s>>>(a);
   mark();
@@ -1076,11 +1085,11 @@ void far_iteration(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, cons
     k_far_eval<<<simt::kCtasPerSm * num_sms, simt::kThreads, eval_smem, s>>>(a, w, 1);
   mark();
   if (a.fast_pivots && wide_row)
-    k_far_row_pivot_f32<kWideThreads, kWideBlocks><<<a.nb, kWideThreads, row_smem_f32(a.ldr, kWideThreads), s>>>(a);
+    k_far_row_pivot_f32<kWideThreads, kWideBlocks><<<wide_grid, kWideThreads, row_smem_f32(a.ldr, kWideThreads), s>>>(a);
   else if (a.fast_pivots)
     k_far_row_pivot_f32<kPivThreads, kPivBlocksF32><<<piv_grid, kPivThreads, row_smem_f32(a.ldr, kPivThreads), s>>>(a);
   else if (wide_row)
-    k_far_row_pivot<double, kWideThreads, kWideBlocks><<<a.nb, kWideThreads, row_smem, s>>>(a);
+    k_far_row_pivot<double, kWideThreads, kWideBlocks><<<wide_grid, kWideThreads, row_smem, s>>>(a);
   else
     k_far_row_pivot<double, kPivThreads, 8><<<piv_grid, kPivThreads, row_smem, s>>>(a);
   mark();
@@ -1126,11 +1135,20 @@ __global__ void k_batch_end(FarArgs a, int* __restrict__ status, int32_t* __rest
 
 }  // namespace
 
+int far_pivot_width(const FarArgs& a, int k, int64_t left, int64_t num_sms) {
+  if (a.mean_rows < kWideMeanRows) return 0;
+  if (2 * left <= 5 * num_sms) return 3;
+  const bool large = a.max_rows > kWideLargeRows &&
+                     (a.fast_pivots ? k >= 8 && left <= 5 * num_sms : k >= 12 && left <= 8 * num_sms);
+  return large ? 2 : 0;
+}
+
 void far_batch_launch(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, const float* student, int* err,
-                      int num_sms, cudaStream_t s, int iters) {
+                      int num_sms, cudaStream_t s, int iters, const std::vector<int>& active) {
   if (a.nb <= 0) return;
   far_batch_start(a, s);
-  for (int q = 0; q < iters; q++) far_iteration(a, w, tcw, student, err, num_sms, s, nullptr);
+  for (int q = 0; q < iters; q++)
+    far_iteration(a, w, tcw, student, err, num_sms, s, nullptr, q, q < (int)active.size() ? active[q] : a.nb);
 }
 
 void far_batch_end(const FarArgs& a, int* status, int32_t* lists, int cap, cudaStream_t s) {
@@ -1140,25 +1158,27 @@ void far_batch_end(const FarArgs& a, int* status, int32_t* lists, int cap, cudaS
 }
 
 int far_batch_plain(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, const float* student, int* err,
-                    int num_sms, int32_t* host_ctr, cudaStream_t s, int known_iters, int* iterations,
-                    FarTimer* timer) {
+                    int num_sms, int32_t* host_ctr, cudaStream_t s, int known_iters, const std::vector<int>& active,
+                    int* iterations, FarTimer* timer) {
   if (a.nb <= 0) return 0;
   far_batch_start(a, s);
   // Without a known bound the counters are read back every kCheck iterations; the kernels of
   // an iteration with no active block return at once.
   constexpr int kCheck = 4;
   const int limit = known_iters > 0 ? known_iters : a.max_iter + 1;
-  int it = 0;
+  int it = 0, left = a.nb;
   bool finished = false;
   while (it < limit && !finished) {
     const int span = known_iters > 0 ? limit : (it + kCheck < limit ? kCheck : limit - it);
-    for (int q = 0; q < span; q++, it++) far_iteration(a, w, tcw, student, err, num_sms, s, timer);
+    for (int q = 0; q < span; q++, it++)
+      far_iteration(a, w, tcw, student, err, num_sms, s, timer, it, it < (int)active.size() ? active[it] : left);
     HIGNN_CUDA(cudaMemcpyAsync(host_ctr, a.ctr, sizeof(int32_t) * kCtrCount, cudaMemcpyDeviceToHost, s));
     HIGNN_CUDA(cudaStreamSynchronize(s));
     if (timer) timer->collect();
     if (host_ctr[kCtrError] != 0)
       throw Error(-5, "ACA: pivot search found no unused row/column (non-finite block entries?)");
-    finished = host_ctr[kCtrRemaining] == 0;
+    left = host_ctr[kCtrRemaining];
+    finished = left == 0;
   }
   if (!finished) throw Error(-5, "ACA did not converge within max_iter iterations");
   if (iterations) *iterations += it;

@@ -85,6 +85,7 @@ struct FarArgs {
   int defer_apply;  // 1: converged blocks are applied later by far_student_check
   int fast_pivots;  // 1: orthogonalisation, pivot search and stopping norms in FP32 (the fast
                     // forms); 0: in FP64, as the restated reference
+  int mean_rows, max_rows;  // of the batch's blocks: mean of |I| and |J|, largest of them (width of the pivot CTAs)
 };
 
 constexpr int kFarSamples = 64;  // sampled entries per block in the student residual check
@@ -93,7 +94,10 @@ constexpr int kFarSamples = 64;  // sampled entries per block in the student res
 // tcw != nullptr -> teacher on the tensor cores; else teacher FP32 SIMT. known_iters > 0:
 // every block stops (converges or is deferred) within that many iterations, so they are
 // launched without reading the counters back in between; 0: counters are read every
-// few iterations. Returns the number of deferred blocks.
+// few iterations. active[k]: blocks expected to be left in iteration k (where it ends: as read back); it
+// chooses the width of the pivot CTAs. Returns the number of deferred blocks.
+// Width of iteration k's pivot CTAs with `left` blocks expected to be left: 1 wide column, 2 wide row pivots.
+int far_pivot_width(const FarArgs& a, int k, int64_t left, int64_t num_sms);
 // Optional per-category timing of a batch: CUDA events around every launch, summed after the
 // batch (milliseconds added to the four totals).
 struct FarTimer {
@@ -106,14 +110,14 @@ struct FarTimer {
 };
 
 int far_batch_plain(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, const float* student, int* err,
-                    int num_sms, int32_t* host_ctr, cudaStream_t s, int known_iters, int* iterations,
-                    FarTimer* timer = nullptr);
+                    int num_sms, int32_t* host_ctr, cudaStream_t s, int known_iters, const std::vector<int>& active,
+                    int* iterations, FarTimer* timer = nullptr);
 
 // Graph form of a batch (no host read-back): its state and `iters` iterations, every block's rank
 // known in advance; far_batch_end folds its counters into `status` and lists the blocks to rerun
 // (see k_batch_end in far_aca.cu).
 void far_batch_launch(const FarArgs& a, const MlpF32& w, const TcWeights* tcw, const float* student, int* err,
-                      int num_sms, cudaStream_t s, int iters);
+                      int num_sms, cudaStream_t s, int iters, const std::vector<int>& active);
 void far_batch_end(const FarArgs& a, int* status, int32_t* lists, int cap, cudaStream_t s);
 // far_student_check without the read-back of the count of blocks sent back to the teacher.
 void far_student_check_launch(const FarArgs& a, const TcWeights& tcw, const float* student, float tol, float* feat,
