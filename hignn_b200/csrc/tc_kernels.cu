@@ -10,7 +10,7 @@
 //               and flushed with one FP64 atomic per particle and component per
 //               pair (src/CloseDot.cpp:245-299).
 //   k_far_tc  : column / row queries of all active ACA blocks, symmetrised into
-//               the FP64 C / Q pools (src/FarDot.cpp:348-458, 672-781).
+//               the C / Q pools (src/FarDot.cpp:348-458, 672-781).
 //   k_eval_tc : M(r) for an array of features.
 #include "common.h"
 #include "kernels.h"
@@ -228,29 +228,37 @@ __device__ __forceinline__ void far_put(tc::Server& sv, const FarArgs& a, int wh
     lo += __popc(m) * step;
     hi = min(hi, lo + step);
   }
+  // The rows' loads depend on one another (block, its state, the pivot, positions): taken step by step for all
+  // of the lane's rows, so that the four chains run at once (700 spheres, one tile per launch: 16.4 instead of 18.2 us,
+  // 131,072 spheres: queries 49.0 instead of 52.0 ms).
+  int b[kParts], loc[kParts];
+  bool in[kParts];
 #pragma unroll
   for (int k = 0; k < kParts; k++) {
     const int g = g0 + 32 * k + sv.lane;
+    in[k] = g < tot;
+    while (in[k] && pre[lo + 1] <= g) lo++;
+    b[k] = a.act[lo];
+    loc[k] = g - pre[lo];
+  }
+  float4 xi[kParts], xj[kParts];
+#pragma unroll
+  for (int k = 0; k < kParts; k++) {
+    const FarBlock& bk = a.blocks[b[k]];
+    const int it = a.state[b[k]].k;
+    const int pivot = (which == 0 ? a.cols : a.rows)[(size_t)b[k] * a.ldr + it];
+    const int own = in[k] ? loc[k] : 0;  // padding rows repeat the block's first
+    xj[k] = a.x[bk.sJ + (which == 0 ? pivot : own)];
+    xi[k] = a.x[bk.sI + (which == 0 ? own : pivot)];
+    c.dst[k] = !in[k] ? -1 : which == 0 ? bk.cOff + (int64_t)it * bk.nI + own : bk.qOff + (int64_t)it * bk.nJ + own;
+  }
+#pragma unroll
+  for (int k = 0; k < kParts; k++) {
     float r[3] = {1.f, 0.f, 0.f};
-    c.dst[k] = -1;
-    if (g < tot) {
-      while (pre[lo + 1] <= g) lo++;
-      const int b = a.act[lo], loc = g - pre[lo];
-      const FarBlock bk = a.blocks[b];
-      const int it = a.state[b].k;
-      float4 xi, xj;
-      if (which == 0) {
-        xj = a.x[bk.sJ + a.cols[(size_t)b * a.ldr + it]];
-        xi = a.x[bk.sI + loc];
-        c.dst[k] = bk.cOff + (int64_t)it * bk.nI + loc;
-      } else {
-        xj = a.x[bk.sJ + loc];
-        xi = a.x[bk.sI + a.rows[(size_t)b * a.ldr + it]];
-        c.dst[k] = bk.qOff + (int64_t)it * bk.nJ + loc;
-      }
-      r[0] = xj.x - xi.x;
-      r[1] = xj.y - xi.y;
-      r[2] = xj.z - xi.z;
+    if (in[k]) {
+      r[0] = xj[k].x - xi[k].x;
+      r[1] = xj[k].y - xi[k].y;
+      r[2] = xj[k].z - xi[k].z;
     }
     sv.put(t, 32 * k + sv.lane, r[0], r[1], r[2]);
   }
@@ -349,7 +357,7 @@ __global__ void __launch_bounds__(tc::kThreads, 1)
           for (int q = 0; q < 9; q++) y[9 * g + q] = M[q];
         }
       }
-          tile = nt;
+      tile = nt;
       have = has_next;
     }
   });
