@@ -29,7 +29,11 @@ struct NearArgs {
   const float4* xJ;  // source positions
   const float4* fJ;
   double* uJ;
+  int64_t evals;  // evaluations of the list where they are few and cut accordingly (plain_tile), or 0
 };
+
+// Evaluations per tile of the plain network for `evals` of them in all.
+int plain_tile(int64_t evals, int num_sms);
 
 void launch_near_simt(const NearArgs& a, const MlpF32& w, int* work_counter, int num_sms, cudaStream_t s);
 // Dense rows with the network in FP64 (kPairSymmetrize items, I side only; dense_f64.cu).

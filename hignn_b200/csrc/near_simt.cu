@@ -24,12 +24,13 @@ struct NearSmem {
   int item;
 };
 
+template <int Rows>
 __global__ void __launch_bounds__(simt::kThreads, simt::kCtasPerSm)
     k_near_simt(NearArgs a, MlpF32 w, int* work_counter) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   NearSmem& s = *reinterpret_cast<NearSmem*>(smem_raw);
   const int t = threadIdx.x, lane = t & 31;
-  const int row = simt::kRows * (t >> 5) + lane;  // lanes 0-15 of a warp: its evaluations of a tile
+  const int row = Rows * (t >> 5) + lane;  // lanes 0 .. Rows - 1 of a warp: its evaluations of a tile
   simt::load_weights(s.mlp, w);
   for (;;) {
     __syncthreads();
@@ -44,16 +45,16 @@ __global__ void __launch_bounds__(simt::kThreads, simt::kCtasPerSm)
     const int i0 = pw.first / pw.nJ, i1 = (end - 1) / pw.nJ;  // targets of the item
     for (int q = 3 * i0 + t; q < 3 * (i1 + 1); q += simt::kThreads) (&s.uI[0][0])[q] = 0.f;
     for (int q = t; q < 3 * pw.nJ; q += simt::kThreads) (&s.uJ[0][0])[q] = 0.f;
-    for (int t0 = pw.first; t0 < end; t0 += simt::kTile) {
+    for (int t0 = pw.first; t0 < end; t0 += simt::kWarps * Rows) {
       const int flat = t0 + row;
-      const bool valid = lane < simt::kRows && flat < end;
+      const bool valid = lane < Rows && flat < end;
       const int i = valid ? flat / pw.nJ : 0, j = valid ? flat - i * pw.nJ : 0;
-      if (lane < simt::kRows) {
+      if (lane < Rows) {
         const float4 xi = __ldg(&a.xI[pw.sI + i]), xj = __ldg(&a.xJ[pw.sJ + j]);
         s.mlp.r[row] = valid ? make_float4(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z, 0.f) : make_float4(1.f, 0.f, 0.f, 0.f);
       }
       __syncthreads();
-      simt::mlp_tile(s.mlp, w);
+      simt::mlp_tile<Rows>(s.mlp, w);
       if (valid) {
         float M[9];
 #pragma unroll
@@ -89,18 +90,33 @@ __global__ void __launch_bounds__(simt::kThreads, simt::kCtasPerSm)
   }
 }
 
+template <int Rows>
+void near_simt(const NearArgs& a, const MlpF32& w, int* work_counter, int num_sms, cudaStream_t stream) {
+  const size_t smem = sizeof(NearSmem);
+  set_max_dynamic_smem(k_near_simt<Rows>, smem, stream);
+  HIGNN_CUDA(cudaMemsetAsync(work_counter, 0, sizeof(int), stream));
+  const int ctas = simt::kCtasPerSm * num_sms;
+  const int grid = a.nwork < ctas ? a.nwork : ctas;
+  k_near_simt<Rows><<<grid, simt::kThreads, smem, stream>>>(a, w, work_counter);
+  HIGNN_CHECK_LAUNCH();
+}
+
 }  // namespace
+
+int plain_tile(int64_t evals, int num_sms) {
+  return simt::kWarps * simt::rows_per_warp(evals, (int64_t)simt::kCtasPerSm * num_sms);
+}
 
 void launch_near_simt(const NearArgs& a, const MlpF32& w, int* work_counter, int num_sms,
                       cudaStream_t stream) {
   if (a.nwork <= 0) return;
-  const size_t smem = sizeof(NearSmem);
-  set_max_dynamic_smem(k_near_simt, smem, stream);
-  HIGNN_CUDA(cudaMemsetAsync(work_counter, 0, sizeof(int), stream));
-  const int ctas = simt::kCtasPerSm * num_sms;
-  const int grid = a.nwork < ctas ? a.nwork : ctas;
-  k_near_simt<<<grid, simt::kThreads, smem, stream>>>(a, w, work_counter);
-  HIGNN_CHECK_LAUNCH();
+  const int tile = a.evals > 0 ? plain_tile(a.evals, num_sms) : simt::kTile;
+  if (tile == simt::kTile / 4)
+    near_simt<simt::kRows / 4>(a, w, work_counter, num_sms, stream);
+  else if (tile == simt::kTile / 2)
+    near_simt<simt::kRows / 2>(a, w, work_counter, num_sms, stream);
+  else
+    near_simt<simt::kRows>(a, w, work_counter, num_sms, stream);
 }
 
 }  // namespace hignn
