@@ -296,26 +296,33 @@ void build_structures(hignn_model* m) {
   // device copies
   HIGNN_CUDA(cudaSetDevice(m->device));
   const int64_t n = m->n;
-  std::vector<float4> x4(n);
-  std::vector<int32_t> perm(n), slot(n);
-  for (int64_t i = 0; i < n; i++) {
-    x4[i] = make_float4(m->xt[3 * i], m->xt[3 * i + 1], m->xt[3 * i + 2], 0.f);
-    perm[i] = (int32_t)m->tree.perm[i];
-    slot[i] = (int32_t)m->inv_perm[i];
+  std::vector<float4> x4;  // the device tree has them, and the permutation, on the device already
+  std::vector<int32_t> perm, slot(n);
+  for (int64_t i = 0; i < n; i++) slot[i] = (int32_t)m->inv_perm[i];
+  if (!on_dev) {
+    x4.resize(n);
+    perm.resize(n);
+    for (int64_t i = 0; i < n; i++) {
+      x4[i] = make_float4(m->xt[3 * i], m->xt[3 * i + 1], m->xt[3 * i + 2], 0.f);
+      perm[i] = (int32_t)m->tree.perm[i];
+    }
   }
   // close work list (src/CloseFarCheck.cpp:298-336 order). Where the pairs are too few to keep every SM
   // busy to the end (two work items in flight per SM, about eight per slot wanted), they are cut into
   // runs of evaluations, whole tiles each; m->close_item0 gives every pair's first item. (601 spheres have 109
   // pairs for 148 SMs; their plain product took 3.65 ms with whole pairs, 2.03 ms with both this and the
-  // faster network; from about 100,000 particles on no pair is cut.)
+  // faster network. No pair is cut where an item has room for two full leaves, 16,384 evaluations: from 3.9e7
+  // evaluations on, some 15,000 particles in leaves of 128.)
   std::vector<hignn::PairWork> work;
   const size_t nclose = m->lists.closeI.size();
-  work.reserve(nclose);
+  work.reserve(nclose + 8 * 2 * m->num_sms);
   int64_t evals = 0;
+  m->max_leaf = 0;
   for (size_t q = 0; q < nclose; q++) {
     const auto& I = m->tree.nodes[m->lists.closeI[q]];
     const auto& J = m->tree.nodes[m->lists.closeJ[q]];
     evals += (I.end - I.start) * (J.end - J.start);
+    m->max_leaf = std::max(m->max_leaf, (int)std::max(I.end - I.start, J.end - J.start));
   }
   const int64_t per_item = item_evals((double)evals, 8 * 2 * m->num_sms);
   m->close_item0.resize(nclose + 1);
@@ -333,8 +340,6 @@ void build_structures(hignn_model* m) {
   }
   m->close_item0[nclose] = (int64_t)work.size();
   m->stats.close_evals = evals;
-  m->max_leaf = 0;
-  for (const auto& w : work) m->max_leaf = std::max(m->max_leaf, std::max(w.nI, w.nJ));
   m->x4.ensure(sizeof(float4) * n);
   m->perm.ensure(sizeof(int32_t) * n);
   m->slot.ensure(sizeof(int32_t) * n);
