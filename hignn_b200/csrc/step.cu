@@ -217,12 +217,13 @@ __device__ __forceinline__ bool is_neighbour(const float4 xi, const float4 xj, d
   return d * d < c2;
 }
 
-constexpr int kNbrWarps = 4;
+constexpr int kNbrThreads = 128;
+constexpr int kNbrLanes = 16;   // lanes per particle
 constexpr int kNbrStage = 256;  // neighbours of a particle sorted in shared memory
 
-// Sorts v[0 .. n - 1] ascending, by one warp: a bitonic network whose comparators all put the smaller value first, so
-// that indices from n on (as if filled with the largest value) need no storage.
-__device__ __forceinline__ void warp_sort(int* v, int n, int lane) {
+// Sorts v[0 .. n - 1] ascending, by the kNbrLanes lanes of `mask`: a bitonic network whose comparators all put the smaller
+// value first, so that indices from n on (as if filled with the largest value) need no storage.
+__device__ __forceinline__ void group_sort(int* v, int n, int lane, unsigned mask) {
   auto order = [&](int a, int b) {
     if (b < n) {
       const int x = v[a], y = v[b];
@@ -230,42 +231,45 @@ __device__ __forceinline__ void warp_sort(int* v, int n, int lane) {
     }
   };
   for (int k = 2; k < 2 * n; k <<= 1) {
-    __syncwarp();
+    __syncwarp(mask);
     const int h = k >> 1;
-    for (int t = lane; t < n; t += 32) {  // pair t of the step that folds runs of k
+    for (int t = lane; t < n; t += kNbrLanes) {  // pair t of the step that folds runs of k
       const int a = (t & ~(h - 1)) * 2 + (t & (h - 1));
       if (a >= n) break;
       order(a, a ^ (k - 1));
     }
     for (int j = h >> 1; j > 0; j >>= 1) {
-      __syncwarp();
-      for (int t = lane; t < n; t += 32) {
+      __syncwarp(mask);
+      for (int t = lane; t < n; t += kNbrLanes) {
         const int a = (t & ~(j - 1)) * 2 + (t & (j - 1));
         if (a >= n) break;
         order(a, a + j);
       }
     }
   }
-  __syncwarp();
+  __syncwarp(mask);
 }
 
 // Neighbours j != i of every i within the cutoff: count (out == nullptr) or write them, ascending,
-// at out[off[i] ..]. One warp per particle: the three cells of a row along x are one run of the sorted items, and the
-// nine runs of a particle are looked through end to end, 32 items at a time. Up to 32 neighbours are ranked in
-// registers, up to kNbrStage sorted in shared memory, more in place. The bound is the latency of the loads behind one
-// another (start, items, x) where particles are few, else the instructions per candidate. Measured on one B200, the whole
-// two-body list: 1,000,000 particles of 8 / 24 / 100 neighbours 1.31 / 2.29 / 7.65 ms, 20,000 of 28 0.18 ms; with one thread per
-// particle, a chain through 27 cells and an insertion in global memory, 1.62 / 3.83 / 23.6 and 0.62 ms; with a warp that
-// walks the nine runs one by one and lets one lane sort more than 32, 2.49 / 3.02 / 36.0 and 0.24 ms.
-__global__ void __launch_bounds__(32 * kNbrWarps)
+// at out[off[i] ..]. Half a warp per particle: the three cells of a row along x are one run of the sorted items, and the
+// nine runs of a particle are looked through end to end, 16 items at a time. Up to 32 neighbours are ranked
+// against one another, up to kNbrStage sorted in shared memory, more in place. The bound is the latency of the loads behind
+// one another (start, items, x) where particles or neighbours are few, else the instructions per candidate.
+// Measured on one B200, the whole two-body list: 1,000,000 particles of 0.2 / 8 / 24 / 100 neighbours 0.67 / 1.31 / 2.45 / 8.3
+// ms, 20,000 of 28 0.20 ms; with one thread per particle, a chain through 27 cells and an insertion in global memory,
+// 0.67 / 1.62 / 3.83 / 23.6 and 0.61 ms; with a whole warp 1.03 / 1.31 / 2.29 / 7.65 and 0.18 ms (most of its lanes idle where
+// neighbours are few), with a warp that walks the runs one by one and sorts in one lane - / 2.49 / 3.02 / 36.0 and 0.24 ms.
+__global__ void __launch_bounds__(kNbrThreads)
     k_neighbours(const float4* __restrict__ x, int64_t n, CellGrid g, const int* __restrict__ start,
                  const int* __restrict__ items, double cutoff, int64_t* __restrict__ count,
                  const int64_t* __restrict__ off, int* __restrict__ out) {
-  __shared__ int stage[kNbrWarps][kNbrStage];
-  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  __shared__ int stage[kNbrThreads / kNbrLanes][kNbrStage];
+  const int64_t i = ((int64_t)blockIdx.x * kNbrThreads + threadIdx.x) / kNbrLanes;
   if (i >= n) return;
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
+  const int64_t deg = out ? off[i + 1] - off[i] : 0;
+  if (out && deg == 0) return;
+  const int lane = threadIdx.x % kNbrLanes, half = threadIdx.x & kNbrLanes;
+  const unsigned mask = 0xffffu << half;
   const float4 xi = x[i];
   const double c2 = radius_sq(cutoff);
   const int3 c = cell_of(xi, g);
@@ -281,42 +285,50 @@ __global__ void __launch_bounds__(32 * kNbrWarps)
   }
   int end = len;
 #pragma unroll
-  for (int o = 1; o < 16; o <<= 1) {
-    const int v = __shfl_up_sync(full, end, o);
+  for (int o = 1; o < kNbrLanes; o <<= 1) {
+    const int v = __shfl_up_sync(mask, end, o, kNbrLanes);
     if (lane >= o) end += v;
   }
-  const int shift = r0 - (end - len), total = __shfl_sync(full, end, 8);
+  const int shift = r0 - (end - len), total = __shfl_sync(mask, end, 8, kNbrLanes);
+  if (!out && total <= 1) {  // the particle alone
+    if (lane == 0) count[i] = 0;
+    return;
+  }
   int ends[8];
 #pragma unroll
-  for (int q = 0; q < 8; q++) ends[q] = __shfl_sync(full, end, q);
-  const int64_t deg = out ? off[i + 1] - off[i] : 0;
+  for (int q = 0; q < 8; q++) ends[q] = __shfl_sync(mask, end, q, kNbrLanes);
   int* dst = out ? out + off[i] : nullptr;
-  int* v = deg <= kNbrStage ? stage[threadIdx.x >> 5] : dst;
+  int* v = deg <= kNbrStage ? stage[threadIdx.x / kNbrLanes] : dst;
   int cnt = 0;
-  for (int k0 = 0; k0 < total; k0 += 32) {
+  for (int k0 = 0; k0 < total; k0 += kNbrLanes) {
     const int k = k0 + lane;
     int run = 0;
 #pragma unroll
     for (int q = 0; q < 8; q++) run += k >= ends[q] ? 1 : 0;
-    const int to = __shfl_sync(full, shift, run);
+    const int to = __shfl_sync(mask, shift, run, kNbrLanes);
     const int j = k < total ? items[k + to] : (int)i;
     const bool hit = j != (int)i && is_neighbour(xi, x[j], c2);
-    const unsigned m = __ballot_sync(full, hit);
+    const unsigned m = (__ballot_sync(mask, hit) >> half) & 0xffffu;
     if (out && hit) v[cnt + __popc(m & ((1u << lane) - 1u))] = j;
     cnt += __popc(m);
   }
   if (count && lane == 0) count[i] = cnt;
   if (!out) return;
-  __syncwarp();
-  if (cnt <= 32) {
-    const int mine = lane < cnt ? v[lane] : 0;
-    int rank = 0;
-    for (int q = 0; q < cnt; q++) rank += __shfl_sync(full, mine, q) < mine ? 1 : 0;
-    if (lane < cnt) dst[rank] = mine;
+  __syncwarp(mask);
+  if (cnt <= 2 * kNbrLanes) {
+    const int a = lane < cnt ? v[lane] : 0, b = lane + kNbrLanes < cnt ? v[lane + kNbrLanes] : 0;
+    int ra = 0, rb = 0;
+    for (int q = 0; q < cnt; q++) {
+      const int w = v[q];
+      ra += w < a ? 1 : 0;
+      rb += w < b ? 1 : 0;
+    }
+    if (lane < cnt) dst[ra] = a;
+    if (lane + kNbrLanes < cnt) dst[rb] = b;
   } else {
-    warp_sort(v, cnt, lane);
+    group_sort(v, cnt, lane, mask);
     if (v != dst)
-      for (int q = lane; q < cnt; q += 32) dst[q] = v[q];
+      for (int q = lane; q < cnt; q += kNbrLanes) dst[q] = v[q];
   }
 }
 
@@ -579,8 +591,8 @@ void launch_morse(const float4* x, int64_t n, const CellList& cl, const MorsePar
 void launch_neighbours(const float4* x, int64_t n, const CellList& cl, double cutoff, int64_t* count,
                        const int64_t* off, int* out, cudaStream_t s) {
   if (n <= 0) return;
-  k_neighbours<<<nblk(32 * n, 32 * kNbrWarps), 32 * kNbrWarps, 0, s>>>(x, n, cl.grid, cl.start.as<int>(),
-                                                                     cl.items.as<int>(), cutoff, count, off, out);
+  k_neighbours<<<nblk(kNbrLanes * n, kNbrThreads), kNbrThreads, 0, s>>>(x, n, cl.grid, cl.start.as<int>(),
+                                                                        cl.items.as<int>(), cutoff, count, off, out);
   HIGNN_CHECK_LAUNCH();
 }
 
