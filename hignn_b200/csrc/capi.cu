@@ -115,7 +115,7 @@ struct hignn_model {
   hignn::BlockLists lists;
   std::vector<float> xt;   // tree order
   std::vector<int64_t> inv_perm;
-  std::vector<int64_t> close_item0;  // first near-field work item of each close pair (size num_close + 1)
+  int64_t close_items = 0;  // near-field work items of this shard's close pairs
   bool tree_ready = false;
   bool lists_sym = true;
   int64_t lists_max_rel = 500000;
@@ -224,6 +224,8 @@ void cut_pair(hignn::PairWork w, int64_t per_item, std::vector<hignn::PairWork>&
   }
 }
 
+void ensure_shard(hignn_model* m);
+
 // Builds the tree and lists of m->xyz and, on a device model, uploads the tree-order positions
 // and the close work list. Everything is built and checked before the model changes: a tree that
 // the device kernels cannot take (a leaf above kMaxLeaf particles, which coincident points can
@@ -307,39 +309,6 @@ void build_structures(hignn_model* m) {
       perm[i] = (int32_t)m->tree.perm[i];
     }
   }
-  // close work list (src/CloseFarCheck.cpp:298-336 order). Where the pairs are too few to keep every SM
-  // busy to the end (two work items in flight per SM, about eight per slot wanted), they are cut into
-  // runs of evaluations, whole tiles each; m->close_item0 gives every pair's first item. (601 spheres have 109
-  // pairs for 148 SMs; their plain product took 3.65 ms with whole pairs, 2.03 ms with both this and the
-  // faster network. No pair is cut where an item has room for two full leaves, 16,384 evaluations: from 3.9e7
-  // evaluations on, some 15,000 particles in leaves of 128.)
-  std::vector<hignn::PairWork> work;
-  const size_t nclose = m->lists.closeI.size();
-  work.reserve(nclose + 8 * 2 * m->num_sms);
-  int64_t evals = 0;
-  m->max_leaf = 0;
-  for (size_t q = 0; q < nclose; q++) {
-    const auto& I = m->tree.nodes[m->lists.closeI[q]];
-    const auto& J = m->tree.nodes[m->lists.closeJ[q]];
-    evals += (I.end - I.start) * (J.end - J.start);
-    m->max_leaf = std::max(m->max_leaf, (int)std::max(I.end - I.start, J.end - J.start));
-  }
-  const int64_t per_item = item_evals((double)evals, 8 * 2 * m->num_sms);
-  m->close_item0.resize(nclose + 1);
-  for (size_t q = 0; q < nclose; q++) {
-    const auto& I = m->tree.nodes[m->lists.closeI[q]];
-    const auto& J = m->tree.nodes[m->lists.closeJ[q]];
-    hignn::PairWork w{};
-    w.sI = (int32_t)I.start;
-    w.nI = (int32_t)(I.end - I.start);
-    w.sJ = (int32_t)J.start;
-    w.nJ = (int32_t)(J.end - J.start);
-    w.flags = (m->use_symmetry && m->lists.closeJ[q] > m->lists.closeI[q]) ? hignn::kPairTransposed : 0;
-    m->close_item0[q] = (int64_t)work.size();
-    cut_pair(w, per_item, work);
-  }
-  m->close_item0[nclose] = (int64_t)work.size();
-  m->stats.close_evals = evals;
   m->x4.ensure(sizeof(float4) * n);
   m->perm.ensure(sizeof(int32_t) * n);
   m->slot.ensure(sizeof(int32_t) * n);
@@ -347,7 +316,6 @@ void build_structures(hignn_model* m) {
   m->u.ensure(sizeof(double) * 3 * n);
   m->io_f.ensure(sizeof(float) * 3 * n);
   m->io_u.ensure(sizeof(float) * 3 * n);
-  m->close_work.ensure(sizeof(hignn::PairWork) * std::max<size_t>(1, work.size()));
   m->counter.ensure(64);
   HIGNN_CUDA(cudaMemcpyAsync(m->slot.p, slot.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, m->stream));
   if (on_dev) {  // tree-order positions and the permutation are already on the device
@@ -358,9 +326,7 @@ void build_structures(hignn_model* m) {
     HIGNN_CUDA(cudaMemcpyAsync(m->x4.p, x4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, m->stream));
     HIGNN_CUDA(cudaMemcpyAsync(m->perm.p, perm.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, m->stream));
   }
-  if (!work.empty())
-    HIGNN_CUDA(cudaMemcpyAsync(m->close_work.p, work.data(), sizeof(hignn::PairWork) * work.size(),
-                               cudaMemcpyHostToDevice, m->stream));
+  ensure_shard(m);
   HIGNN_CUDA(cudaStreamSynchronize(m->stream));
   m->tree_ready = true;
 }
@@ -385,6 +351,41 @@ void balanced_range(const std::vector<double>& cost, int rank, int world, int64_
   *hi = std::max(*lo, std::min<int64_t>(cut(rank + 1), (int64_t)n));
 }
 
+// The near-field work list of this shard's close pairs (src/CloseFarCheck.cpp:298-336 order). Where the pairs are too
+// few to keep every SM busy to the end (two work items in flight per SM, about eight per slot wanted), they are cut
+// into runs of evaluations, whole tiles each. (601 spheres have 109 pairs for 148 SMs; their plain product took
+// 3.65 ms with whole pairs, 2.03 ms with both this and the faster network; a 64th of 20,000 clustered spheres, 74 pairs
+// on the tensor cores, 0.18 ms, 0.64 ms cut as the whole list would be. No pair is cut where an item has room for two full leaves, 16,384 evaluations: from
+// 3.9e7 evaluations on, some 15,000 particles in leaves of 128.)
+void upload_close_work(hignn_model* m) {
+  int64_t evals = 0;
+  for (int64_t q = m->sh_c0; q < m->sh_c1; q++) {
+    const auto& I = m->tree.nodes[m->lists.closeI[q]];
+    const auto& J = m->tree.nodes[m->lists.closeJ[q]];
+    evals += (I.end - I.start) * (J.end - J.start);
+  }
+  const int64_t per_item = item_evals((double)evals, 8 * 2 * m->num_sms);
+  std::vector<hignn::PairWork> work;
+  work.reserve(m->sh_c1 - m->sh_c0 + 8 * 2 * m->num_sms);
+  for (int64_t q = m->sh_c0; q < m->sh_c1; q++) {
+    const auto& I = m->tree.nodes[m->lists.closeI[q]];
+    const auto& J = m->tree.nodes[m->lists.closeJ[q]];
+    hignn::PairWork w{};
+    w.sI = (int32_t)I.start;
+    w.nI = (int32_t)(I.end - I.start);
+    w.sJ = (int32_t)J.start;
+    w.nJ = (int32_t)(J.end - J.start);
+    w.flags = (m->use_symmetry && m->lists.closeJ[q] > m->lists.closeI[q]) ? hignn::kPairTransposed : 0;
+    cut_pair(w, per_item, work);
+  }
+  m->close_items = (int64_t)work.size();
+  m->close_work.ensure(sizeof(hignn::PairWork) * std::max<size_t>(1, work.size()));
+  if (work.empty()) return;
+  HIGNN_CUDA(cudaMemcpyAsync(m->close_work.p, work.data(), sizeof(hignn::PairWork) * work.size(), cudaMemcpyHostToDevice,
+                             m->stream));
+  HIGNN_CUDA(cudaStreamSynchronize(m->stream));
+}
+
 // The shard of this model: close pairs balanced by |I||J| evaluations, far pairs by
 // (|I| + |J|) min(kmax, 32) (query rows times a typical rank), contiguous in list order as the
 // reference's ranks take interleaved shares of the same lists (src/CloseFarCheck.cpp:309,394).
@@ -407,6 +408,10 @@ void ensure_shard(hignn_model* m) {
   int64_t evals = 0;
   for (int64_t q = m->sh_c0; q < m->sh_c1; q++) evals += (int64_t)cc[q];
   m->stats.close_evals = evals;
+  m->max_leaf = 0;
+  for (int64_t L : m->lists.leaves)
+    m->max_leaf = std::max(m->max_leaf, (int)(m->tree.nodes[L].end - m->tree.nodes[L].start));
+  if (m->device >= 0) upload_close_work(m);
   m->shard_ready = true;
 }
 
@@ -927,9 +932,8 @@ void far_field(hignn_model* m) {
 void near_field(hignn_model* m) {
   hignn::NearArgs a{};
   ensure_shard(m);
-  const int64_t i0 = m->close_item0[m->sh_c0], i1 = m->close_item0[m->sh_c1];
-  a.work = m->close_work.as<hignn::PairWork>() + i0;
-  a.nwork = (int)(i1 - i0);
+  a.work = m->close_work.as<hignn::PairWork>();
+  a.nwork = (int)m->close_items;
   a.xI = a.xJ = m->x4.as<float4>();
   a.fI = a.fJ = m->f4.as<float4>();
   a.uI = a.uJ = m->u.as<double>();
@@ -1040,8 +1044,7 @@ uint64_t graph_signature(hignn_model* m) {
   mix((uint64_t)m->max_iter);
   mix((uint64_t)m->use_symmetry);
   mix((uint64_t)m->has_student);
-  mix((uint64_t)m->close_item0[m->sh_c0]);
-  mix((uint64_t)m->close_item0[m->sh_c1]);
+  mix((uint64_t)m->close_items);
   mix((uint64_t)m->batches.size());
   for (const auto& bt : m->batches) {
     mix(((uint64_t)bt.b0 << 40) ^ ((uint64_t)bt.b1 << 16) ^ (uint64_t)bt.iters);
