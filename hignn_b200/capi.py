@@ -40,6 +40,9 @@ P_RANK_HINT_OFFSET = 107
 P_TREE_DEVICE = 108
 P_GRAPH = 109
 P_KEEP_RANKS = 110
+# counters of hignn_near_wait_profile: cycles that the issuing, epilogue and tile-server warps spent in each wait
+NEAR_WAIT_SLOTS = {0: "mma_weights", 1: "mma_accumulator_read", 2: "mma_half_in_a2", 8: "epi_features",
+                   9: "epi_layer2_acc", 10: "server_outputs", 11: "epi_a2_free", 12: "epi_total_warp0", 13: "tiles"}
 DENSE_F64 = 64  # hignn_dense_rows precision: the network in FP64
 
 STUDENT_PARAMS = 2537
@@ -384,10 +387,7 @@ class Model:
         """Wait cycles of the tensor-core near field by barrier (HIGNN_P_TIMING >= 3), then reset."""
         c = (C.c_uint64 * 16)()
         check(lib.hignn_near_wait_profile(self._h, c))
-        names = {0: "mma_first_features", 1: "mma_a1", 2: "mma_q0_in_a2", 3: "mma_d3_free", 4: "mma_q1_in_a2",
-                 5: "mma_q2_in_a2", 6: "mma_next_features", 7: "mma_q3_in_a2", 8: "epi_layer1_acc",
-                 9: "epi_layer2_acc", 10: "epi_layer3_acc", 11: "epi_a2_free", 12: "epi_total_warp0", 13: "tiles"}
-        return {names[i]: int(c[i]) for i in names}
+        return {name: int(c[i]) for i, name in NEAR_WAIT_SLOTS.items()}
 
     def get_student(self):
         p = np.empty(STUDENT_PARAMS, np.float32)
