@@ -379,6 +379,7 @@ void upload_close_work(hignn_model* m) {
     cut_pair(w, per_item, work);
   }
   m->close_items = (int64_t)work.size();
+  HIGNN_CUDA(cudaSetDevice(m->device));
   m->close_work.ensure(sizeof(hignn::PairWork) * std::max<size_t>(1, work.size()));
   if (work.empty()) return;
   HIGNN_CUDA(cudaMemcpyAsync(m->close_work.p, work.data(), sizeof(hignn::PairWork) * work.size(), cudaMemcpyHostToDevice,

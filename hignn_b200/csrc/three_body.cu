@@ -26,8 +26,10 @@
 // The weights (1.6 MB of FP16) stream through a five-deep ring of 32 KB shared-memory stages,
 // filled by bulk copies from a host-built image laid out in the order the MMAs consume it.
 //
-// The MMA warp runs its loop warp-uniformly and one elected lane issues, and a wait that is already over reads
-// no clock: 9.95 -> 8.70 ms for 4.41 M triplets (0.49 of the measured bf16 peak). One arrival per
+// The MMA warp runs its loop warp-uniformly and one elected lane issues, and an epilogue's wait that is already over
+// reads no clock: 9.95 -> 8.70 ms for 4.41 M triplets in a short run (0.49 of the measured bf16 peak; 9.6 ms with many calls
+// in a row). The MMA and producer warps do read the clock around every wait, for the wait profile, which is always kept;
+// reading it only on request was slower (9.62 -> 10.06 ms, other code around the waits). One arrival per
 // epilogue warp instead of one per thread was slower (15 ms: the compiler then spills twice as much around the
 // epilogue's constants).
 //
@@ -81,7 +83,7 @@ static_assert(sizeof(TbConst) + 128 <= 32764, "three-body kernel parameters exce
 
 __device__ __forceinline__ bool wait_bar(uint64_t* b, uint32_t parity, int* abort_flag, int* err, int code,
                                          bool honour_abort = true) {
-  if (tc::mbar_try(b, parity)) return true;  // no clock read where the wait is already over
+  if (tc::mbar_try(b, parity)) return true;  // before the clock is read for the timeout
   const long long t0 = clock64();
   while (!mbar_try_sleep(b, parity, 20000u)) {
     if (honour_abort && *(volatile int*)abort_flag) return false;
